@@ -63,14 +63,17 @@ enum { MA_B200_F32 = 0, MA_B200_BF16 = 1, MA_B200_F16 = 2 };
  *                  (2T launches; masks and padding handled)
  *   HEAD_FUSED     one CTA per head, one iteration (T = 1), block size and count <= 32, D <= 64,
  *                  the head's Q, K, V, al and y together within 227 KB of shared memory: both
- *                  stages in one launch, HBM sees Q, K, V once and the result once (1 launch) */
+ *                  stages in one launch, HBM sees Q, K, V once and the result once (1 launch)
+ *   TF32X3         the WARP_MMA stage kernels on f32 tensors, block size and block count up to 128,
+ *                  D <= 80 (multiple of 8): every operand split into two tf32 parts (2T launches) */
 enum {
   MA_B200_KERNEL_AUTO = 0,
   MA_B200_KERNEL_GENERIC = 1,
   MA_B200_KERNEL_TCGEN05 = 2,
   MA_B200_KERNEL_TCGEN05_STAGED = 3, /* (4 is not in use) */
   MA_B200_KERNEL_WARP_MMA = 5,
-  MA_B200_KERNEL_HEAD_FUSED = 6
+  MA_B200_KERNEL_HEAD_FUSED = 6,
+  MA_B200_KERNEL_TF32X3 = 7
 };
 
 typedef struct ma_b200_tensor {

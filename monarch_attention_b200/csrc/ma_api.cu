@@ -42,7 +42,7 @@ int validate(const ma_b200_problem* p, bool need_pointers) {
     return fail(MA_B200_INVALID_ARGUMENT, "unknown dtype");
   if (!(p->qk_dtype == p->v_dtype || p->v_dtype == MA_B200_F32))
     return fail(MA_B200_UNSUPPORTED, "v_dtype must equal qk_dtype or be f32");
-  if (p->kernel < MA_B200_KERNEL_AUTO || p->kernel > MA_B200_KERNEL_HEAD_FUSED || p->kernel == 4)
+  if (p->kernel < MA_B200_KERNEL_AUTO || p->kernel > MA_B200_KERNEL_TF32X3 || p->kernel == 4)
     return fail(MA_B200_INVALID_ARGUMENT, "unknown kernel family");
   if ((long long)p->E * p->H > 0x7fffffffLL / 2) return fail(MA_B200_INVALID_ARGUMENT, "E*H too large");
   if (need_pointers) {
@@ -98,10 +98,17 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, int* kernel)
   const bool head_ok = ma::head_fused_supported(g, p->qk_dtype, p->v_dtype, &why_h);
   if (p->kernel == MA_B200_KERNEL_HEAD_FUSED && !head_ok)
     return fail(MA_B200_UNSUPPORTED, std::string("one-CTA-per-head kernel cannot run this problem: ") + why_h);
+  const char* why_x = "";
+  const bool tf32_ok = ma::tf32x3_supported(g, p->qk_dtype, p->v_dtype, &why_x);
+  if (p->kernel == MA_B200_KERNEL_TF32X3 && !tf32_ok)
+    return fail(MA_B200_UNSUPPORTED, std::string("fp32 tensor-core path cannot run this problem: ") + why_x);
+  // Heads narrower than 24 leave most of a 16-wide contraction step of the fp32 tensor path padded or give it one
+  // step per tile; the thread-per-logit kernels are as fast there.
+  const bool tf32_pays = tf32_ok && g.D >= 24;
   if (p->kernel == MA_B200_KERNEL_AUTO)
     // (the one-CTA-per-head kernel is selectable but not preferred: on the ViT / RoBERTa shapes it
     // measured slower than the two staged launches - these tiny tiles are instruction-bound)
-    *kernel = tc_ok ? MA_B200_KERNEL_TCGEN05 : (warp_ok ? MA_B200_KERNEL_WARP_MMA : MA_B200_KERNEL_GENERIC);
+    *kernel = tc_ok ? MA_B200_KERNEL_TCGEN05 : (warp_ok ? MA_B200_KERNEL_WARP_MMA : (tf32_pays ? MA_B200_KERNEL_TF32X3 : MA_B200_KERNEL_GENERIC));
   else *kernel = p->kernel;
   if (*kernel == MA_B200_KERNEL_GENERIC) {
     const size_t need = ma::generic_stage_smem_bytes(g, g.B > g.M ? ma::kStageRight : ma::kStageLeft);
@@ -162,9 +169,13 @@ int run_forward(const ma_b200_problem* p, void* workspace, size_t workspace_byte
   auto cuda_fail = [&](cudaError_t e, const char* what) {
     return fail(MA_B200_CUDA_ERROR, std::string(what) + ": " + cudaGetErrorString(e));
   };
-  // status word and the stage-completion counters start at zero
-  cudaError_t ce = cudaMemsetAsync(ws + L.status, 0, L.ar - L.status, stream);
-  if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(status, counters)");
+  // Status word and stage-completion counters start at zero.  The stage kernels that wait for nothing clear the
+  // status word themselves: a memset in front of them is 1.5 us on the stream, as much as a small kernel.
+  cudaError_t ce = cudaSuccess;
+  if (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3) {
+    ce = cudaMemsetAsync(ws + L.status, 0, L.ar - L.status, stream);
+    if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(status, counters)");
+  }
   int* counters = reinterpret_cast<int*>(ws + L.counters);
 
   ma::TcPlan plan_store;
@@ -188,7 +199,8 @@ int run_forward(const ma_b200_problem* p, void* workspace, size_t workspace_byte
     cudaError_t e;
     if (L.kernel == MA_B200_KERNEL_TCGEN05_STAGED)
       e = ma::launch_fused(plan, g, counters, stage_idx, stage_idx + 1, 0, stream);
-    else if (L.kernel == MA_B200_KERNEL_WARP_MMA) e = ma::launch_warp_stage(g, p->qk_dtype, kind, first, stream);
+    else if (L.kernel == MA_B200_KERNEL_WARP_MMA || L.kernel == MA_B200_KERNEL_TF32X3)
+      e = ma::launch_warp_stage(g, p->qk_dtype, kind, first, stream);
     else e = ma::launch_generic_stage(g, p->qk_dtype, p->v_dtype, kind, first, stream);
     ++stage_idx;
     if (ev != nullptr) cudaEventRecord(ev[stage_idx], stream);

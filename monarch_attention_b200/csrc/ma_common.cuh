@@ -73,8 +73,10 @@ cudaError_t launch_generic_stage(const Geometry& g, int qk_dtype, int v_dtype, S
                                  cudaStream_t stream);
 size_t generic_stage_smem_bytes(const Geometry& g, StageKind kind);
 
-// Warp-level tensor-core stage kernels (16-bit, block size and count <= 128, D <= 80).
+// Warp-level tensor-core stage kernels (block size and count <= 256, D <= 80).
 bool warp_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
+// The same kernels on fp32 tensors (products of split operands on the tf32 tensor path).
+bool tf32x3_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
 cudaError_t launch_warp_stage(const Geometry& g, int qk_dtype, StageKind kind, bool first, cudaStream_t stream);
 // Whole head per CTA, both stages of a one-iteration call in one launch (state in shared memory).
 bool head_fused_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);

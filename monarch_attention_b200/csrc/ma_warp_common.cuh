@@ -1,0 +1,268 @@
+// Warp-level building blocks shared by the stage kernels (ma_warp.cu) and the backward kernels (ma_backward.cu):
+// ldmatrix / mma.sync wrappers, the asynchronous tile loader, and the 16 x 16 fragment operations of one
+// element type.
+#pragma once
+
+#include "ma_common.cuh"
+
+namespace ma {
+namespace {
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void ldsm_x2(uint32_t addr, uint32_t (&r)[2]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm_x2_trans(uint32_t addr, uint32_t (&r)[2]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+
+template <typename T>
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]);
+template <>
+__device__ __forceinline__ void mma16816<__nv_bfloat16>(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+               "{%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+template <>
+__device__ __forceinline__ void mma16816<__half>(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+               "{%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+template <typename T>
+__device__ __forceinline__ uint32_t pack_pair(float lo, float hi);
+template <>
+__device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float lo, float hi) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+template <>
+__device__ __forceinline__ uint32_t pack_pair<__half>(float lo, float hi) {
+  __half2 v = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+
+__device__ __forceinline__ float quad_max(float v) {
+  v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+  return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+}
+__device__ __forceinline__ float quad_sum(float v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
+// Copies `rows` rows of `width` elements (a multiple of 8) into a shared tile with row
+// pitch `pitch` elements, zero-filling rows that do not exist, columns past width and rows
+// [rows, rpad).  Threads tid of nthreads cooperate.  The copies are asynchronous (cp.async, 16 bytes
+// each, zero-fill by giving a source size of 0): a thread queues all of its pieces without waiting;
+// tiles_commit_and_wait() must be called before the tile is read.
+// Every source these kernels have is an arithmetic progression of rows: row r comes from element
+// offset (n0 + r*nstep)*row_stride of `base` and exists iff r < rows and 0 <= n0 + r*nstep < n_limit
+// (token index inside the sequence; for the dense state tensors n0 = 0, nstep = 1, n_limit = rows).
+// Row, column chunk, token index and source offset are carried from one 16-byte piece to the next
+// with additions only.
+template <typename T, int CHUNKS>  // CHUNKS: 16-byte pieces of a padded row
+__device__ __forceinline__ void load_rows(T* tile, int pitch, int rows, int rpad, int width, const T* base, int n0,
+                                          int nstep, int n_limit, long long row_stride, int tid, int nthreads,
+                                          const void* any_valid_global) {
+  constexpr int kPer = 16 / (int)sizeof(T);  // elements of a piece
+  int r = tid / CHUNKS, c = tid - r * CHUNKS;
+  const int dr = nthreads / CHUNKS, dc = nthreads - dr * CHUNKS;
+  int n = n0 + r * nstep;
+  const T* src = base + (long long)n * row_stride;
+  uint32_t dst = smem_addr(tile + r * pitch);
+  const int dn = dr * nstep;
+  const long long dsrc = (long long)dn * row_stride, step1 = (long long)nstep * row_stride;
+  const uint32_t ddst = (uint32_t)(dr * pitch) * (uint32_t)sizeof(T), dst1 = (uint32_t)pitch * (uint32_t)sizeof(T);
+  while (r < rpad) {
+    const bool ok = r < rows && c * kPer < width && (unsigned)n < (unsigned)n_limit;
+    const void* gsrc = ok ? static_cast<const void*>(src + c * kPer) : any_valid_global;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(c << 4)), "l"(gsrc),
+                 "r"(ok ? 16u : 0u)
+                 : "memory");
+    c += dc; r += dr; n += dn; src += dsrc; dst += ddst;
+    if (c >= CHUNKS) { c -= CHUNKS; ++r; n += nstep; src += step1; dst += dst1; }
+  }
+}
+__device__ __forceinline__ void tiles_commit_and_wait() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// The first kernel of a call zeroes the workspace's status word, so that no separate clear has to be queued.
+__device__ __forceinline__ void clear_status(const Geometry& g) {
+  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) *g.status = 0;
+}
+
+__device__ __forceinline__ bool pos_valid(const Geometry& g, int e, int p) {
+  const int n = p - g.pad_off;
+  if (n < 0 || n >= g.N) return false;
+  return g.mask == nullptr || g.mask[(long long)e * g.mask_se + n] != 0;
+}
+// Row of a user tensor for padded position p, given the (e, h) base pointer: nullptr for padding.
+template <typename T>
+__device__ __forceinline__ const T* head_base(const View4& t, int e, int h) {
+  return reinterpret_cast<const T*>(t.ptr) + (long long)e * t.se + (long long)h * t.sh;
+}
+// ---------------------------------------------------------------------------------------------------
+// Contractions of one warp on 16 x 16 pieces of one element type: A (16 x 16) times B (16 x 16, as two n8 tiles)
+// into two m16n8 fp32 accumulator tiles.  16-bit types: one m16n8k16 per n8 tile.  fp32: operands split into a
+// tf32 part and the tf32 of the remainder, three m16n8k8 per n8 tile and k8 step (small products first), which keeps
+// about 22 bits of every operand; the plain fp32 pipes would need 32 x as many instructions for the same tile.
+// Accumulator element layout (both): c[0], c[1] = row lane/4, columns 2*(lane%4), +1; c[2], c[3] = row + 8.
+// ---------------------------------------------------------------------------------------------------
+template <typename T>
+struct Tile {
+  struct A { uint32_t r[4]; };
+  struct B { uint32_t r[4]; };
+  // A[m][k] = s[m * pitch + k]
+  static __device__ __forceinline__ void load_a(A& a, const T* s, int pitch, int lane) {
+    ldsm_x4(smem_addr(s + ((lane & 7) + ((lane >> 3) & 1) * 8) * pitch + (lane >> 4) * 8), a.r);
+  }
+  // A[m][k] = s[k * pitch + m]
+  static __device__ __forceinline__ void load_a_t(A& a, const T* s, int pitch, int lane) {
+    ldsm_x4_trans(smem_addr(s + ((lane & 7) + (lane >> 4) * 8) * pitch + ((lane >> 3) & 1) * 8), a.r);
+  }
+  // B[k][n] = s[n * pitch + k]
+  static __device__ __forceinline__ void load_b_nk(B& b, const T* s, int pitch, int lane) {
+    ldsm_x4(smem_addr(s + ((lane & 7) + (lane >> 4) * 8) * pitch + ((lane >> 3) & 1) * 8), b.r);
+  }
+  // B[k][n] = s[k * pitch + n]
+  static __device__ __forceinline__ void load_b_kn(B& b, const T* s, int pitch, int lane) {
+    ldsm_x4_trans(smem_addr(s + ((lane & 7) + ((lane >> 3) & 1) * 8) * pitch + (lane >> 4) * 8), b.r);
+  }
+  static __device__ __forceinline__ void from_acc(A& a, const float (&c0)[4], const float (&c1)[4]) {
+    a.r[0] = pack_pair<T>(c0[0], c0[1]);
+    a.r[1] = pack_pair<T>(c0[2], c0[3]);
+    a.r[2] = pack_pair<T>(c1[0], c1[1]);
+    a.r[3] = pack_pair<T>(c1[2], c1[3]);
+  }
+  static __device__ __forceinline__ void mma(float (&c0)[4], float (&c1)[4], const A& a, const B& b) {
+    const uint32_t b0[2] = {b.r[0], b.r[1]}, b1[2] = {b.r[2], b.r[3]};
+    mma16816<T>(c0, a.r, b0);
+    mma16816<T>(c1, a.r, b1);
+  }
+  static __device__ __forceinline__ void store_pair(T* p, float lo, float hi) {
+    *reinterpret_cast<uint32_t*>(p) = pack_pair<T>(lo, hi);
+  }
+};
+
+__device__ __forceinline__ void mma1688_tf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                             uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+               "{%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// The k index inside a k8 step is permuted so that a step's columns are those of one accumulator tile: k = t is
+// column 2t, k = t + 4 is column 2t + 1 (t = lane % 4), for A and B alike.
+template <>
+struct Tile<float> {
+  struct A { float hi[8], lo[8]; };  // [step][a0..a3]
+  struct B { float hi[8], lo[8]; };  // [n8 tile][step][b0, b1]
+  static __device__ __forceinline__ void split(float x, float& hi, float& lo) {
+    // round to nearest at 11 bits, twice (the tensor path ignores the bits below, so the remainder's need not be
+    // cleared); rounding instead of cutting takes the result's error from 3e-6 to 5e-7, the plain fp32 kernels' own
+    hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+    lo = __uint_as_float(__float_as_uint(x - hi) + 0x1000u);
+  }
+  static __device__ __forceinline__ void load_a(A& a, const float* s, int pitch, int lane) {
+    const float* p = s + (lane >> 2) * pitch + 2 * (lane & 3);
+#pragma unroll
+    for (int st = 0; st < 2; ++st) {
+      const float2 x = *reinterpret_cast<const float2*>(p + 8 * st);
+      const float2 y = *reinterpret_cast<const float2*>(p + 8 * pitch + 8 * st);
+      split(x.x, a.hi[4 * st], a.lo[4 * st]);
+      split(y.x, a.hi[4 * st + 1], a.lo[4 * st + 1]);
+      split(x.y, a.hi[4 * st + 2], a.lo[4 * st + 2]);
+      split(y.y, a.hi[4 * st + 3], a.lo[4 * st + 3]);
+    }
+  }
+  static __device__ __forceinline__ void load_a_t(A& a, const float* s, int pitch, int lane) {
+    const float* p = s + 2 * (lane & 3) * pitch + (lane >> 2);
+#pragma unroll
+    for (int st = 0; st < 2; ++st) {
+      split(p[(8 * st) * pitch], a.hi[4 * st], a.lo[4 * st]);
+      split(p[(8 * st) * pitch + 8], a.hi[4 * st + 1], a.lo[4 * st + 1]);
+      split(p[(8 * st + 1) * pitch], a.hi[4 * st + 2], a.lo[4 * st + 2]);
+      split(p[(8 * st + 1) * pitch + 8], a.hi[4 * st + 3], a.lo[4 * st + 3]);
+    }
+  }
+  static __device__ __forceinline__ void load_b_nk(B& b, const float* s, int pitch, int lane) {
+    const float* p = s + (lane >> 2) * pitch + 2 * (lane & 3);
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int st = 0; st < 2; ++st) {
+        const float2 x = *reinterpret_cast<const float2*>(p + 8 * n * pitch + 8 * st);
+        split(x.x, b.hi[4 * n + 2 * st], b.lo[4 * n + 2 * st]);
+        split(x.y, b.hi[4 * n + 2 * st + 1], b.lo[4 * n + 2 * st + 1]);
+      }
+  }
+  static __device__ __forceinline__ void load_b_kn(B& b, const float* s, int pitch, int lane) {
+    const float* p = s + 2 * (lane & 3) * pitch + (lane >> 2);
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int st = 0; st < 2; ++st) {
+        split(p[(8 * st) * pitch + 8 * n], b.hi[4 * n + 2 * st], b.lo[4 * n + 2 * st]);
+        split(p[(8 * st + 1) * pitch + 8 * n], b.hi[4 * n + 2 * st + 1], b.lo[4 * n + 2 * st + 1]);
+      }
+  }
+  static __device__ __forceinline__ void from_acc(A& a, const float (&c0)[4], const float (&c1)[4]) {
+#pragma unroll
+    for (int st = 0; st < 2; ++st) {
+      const float(&c)[4] = st == 0 ? c0 : c1;
+      split(c[0], a.hi[4 * st], a.lo[4 * st]);
+      split(c[2], a.hi[4 * st + 1], a.lo[4 * st + 1]);
+      split(c[1], a.hi[4 * st + 2], a.lo[4 * st + 2]);
+      split(c[3], a.hi[4 * st + 3], a.lo[4 * st + 3]);
+    }
+  }
+  static __device__ __forceinline__ void mma_part(float (&c)[4], const float* a, const float* b) {
+    mma1688_tf32(c, __float_as_uint(a[0]), __float_as_uint(a[1]), __float_as_uint(a[2]), __float_as_uint(a[3]),
+                 __float_as_uint(b[0]), __float_as_uint(b[1]));
+  }
+  // The tensor path aligns a step's products and its accumulator input to the largest of them and cuts the rest
+  // off, so a long chain of steps on one accumulator drifts.  Every 16 products therefore start from zero (small
+  // parts first) and are added to the running sum by an ordinary rounded addition.
+  static __device__ __forceinline__ void mma(float (&c0)[4], float (&c1)[4], const A& a, const B& b) {
+    float t0[4] = {0.f, 0.f, 0.f, 0.f}, t1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int st = 0; st < 2; ++st) {
+      mma_part(t0, a.lo + 4 * st, b.hi + 2 * st);
+      mma_part(t1, a.lo + 4 * st, b.hi + 4 + 2 * st);
+      mma_part(t0, a.hi + 4 * st, b.lo + 2 * st);
+      mma_part(t1, a.hi + 4 * st, b.lo + 4 + 2 * st);
+    }
+#pragma unroll
+    for (int st = 0; st < 2; ++st) {
+      mma_part(t0, a.hi + 4 * st, b.hi + 2 * st);
+      mma_part(t1, a.hi + 4 * st, b.hi + 4 + 2 * st);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { c0[i] += t0[i]; c1[i] += t1[i]; }
+  }
+  static __device__ __forceinline__ void store_pair(float* p, float lo, float hi) {
+    *reinterpret_cast<float2*>(p) = make_float2(lo, hi);
+  }
+};
+
+}  // namespace
+}  // namespace ma
