@@ -135,6 +135,22 @@ MA_B200_API int ma_b200_forward(const ma_b200_problem* p, void* workspace, size_
 MA_B200_API int ma_b200_forward_timed(const ma_b200_problem* p, void* workspace, size_t workspace_bytes, void* stream,
                           float* stage_ms, int32_t n_stage_ms);
 
+/* Gradients of a forward call: grad_out is the gradient of the result (read; strides of 0 allowed), dq, dk, dv are
+ * written (a NULL pointer: not wanted).  grad_out and dv have v_dtype, dq and dk have qk_dtype; rows of D elements with
+ * unit inner stride on 16-byte boundaries. */
+typedef struct ma_b200_gradients {
+  ma_b200_tensor grad_out, dq, dk, dv;
+} ma_b200_gradients;
+
+/* Enqueue the backward pass of `p` on `stream` (p->out and p->kernel are ignored).  The stage inputs are recomputed
+ * from q, k, v, so nothing has to be kept from the forward call.  Takes the problems of the WARP_MMA and TF32X3
+ * kernels with block size and block count up to 128 (64 in fp32); ma_b200_backward_workspace_bytes returns 0 for others (the caller
+ * then differentiates a recomputation).
+ * reference: autograd through ma/ma_torch.py:10-108, which is how the reference trains. */
+MA_B200_API size_t ma_b200_backward_workspace_bytes(const ma_b200_problem* p);
+MA_B200_API int ma_b200_backward(const ma_b200_problem* p, const ma_b200_gradients* g, void* workspace,
+                                 size_t workspace_bytes, void* stream);
+
 /* Synchronise `stream` and read the device-side status flag of the last forward that used
  * this workspace: MA_B200_OK or MA_B200_DEVICE_WAIT_EXPIRED. */
 MA_B200_API int ma_b200_device_status(void* workspace, void* stream);

@@ -26,6 +26,7 @@ EXPORTS = (
     "ma_b200_forward_static_scratch", "ma_b200_static_scratch_bytes", "ma_b200_static_scratch_last_error",
     "ma_b200_host_scratch_bytes", "ma_b200_forward_host", "ma_b200_forward_host_streamed", "ma_b200_host_last_error",
     "ma_b200_poll_device_status", "ma_b200_selftest_wait_expiry", "ma_b200_selftest_generic_general_form",
+    "ma_b200_backward_workspace_bytes", "ma_b200_backward",
 )
 
 
@@ -42,6 +43,10 @@ class Problem(C.Structure):
         ("q", Tensor4), ("k", Tensor4), ("v", Tensor4), ("out", Tensor4),
         ("mask", C.c_void_p), ("mask_stride_e", C.c_int64),
     ]
+
+
+class Gradients(C.Structure):
+    _fields_ = [(n, Tensor4) for n in ("grad_out", "dq", "dk", "dv")]
 
 
 class WorkspaceLayout(C.Structure):
@@ -71,6 +76,10 @@ def load() -> C.CDLL:
     lib.ma_b200_forward.restype = C.c_int
     lib.ma_b200_forward_timed.argtypes = [pp, C.c_void_p, C.c_size_t, C.c_void_p, C.POINTER(C.c_float), C.c_int32]
     lib.ma_b200_forward_timed.restype = C.c_int
+    lib.ma_b200_backward_workspace_bytes.argtypes = [pp]
+    lib.ma_b200_backward_workspace_bytes.restype = C.c_size_t
+    lib.ma_b200_backward.argtypes = [pp, C.POINTER(Gradients), C.c_void_p, C.c_size_t, C.c_void_p]
+    lib.ma_b200_backward.restype = C.c_int
     lib.ma_b200_device_status.argtypes = [C.c_void_p, C.c_void_p]
     lib.ma_b200_device_status.restype = C.c_int
     lib.ma_b200_poll_device_status.argtypes = [C.c_int]

@@ -271,6 +271,51 @@ int ma_b200_forward_timed(const ma_b200_problem* p, void* workspace, size_t work
   return run_forward(p, workspace, workspace_bytes, stream, stage_ms, n_stage_ms);
 }
 
+size_t ma_b200_backward_workspace_bytes(const ma_b200_problem* p) {
+  if (validate(p, false) != MA_B200_OK) return 0;
+  const ma::Geometry g = make_geometry(p);
+  const char* why = "";
+  if (!ma::backward_supported(g, p->qk_dtype, p->v_dtype, &why)) {
+    fail(MA_B200_UNSUPPORTED, std::string("backward kernels cannot run this problem: ") + why);
+    return 0;
+  }
+  return ma::backward_layout(g, p->qk_dtype).total;
+}
+
+int ma_b200_backward(const ma_b200_problem* p, const ma_b200_gradients* gr, void* workspace, size_t workspace_bytes,
+                     void* stream) {
+  if (p == nullptr || gr == nullptr) return fail(MA_B200_INVALID_ARGUMENT, "problem or gradients is NULL");
+  ma_b200_problem q = *p;
+  q.out = gr->grad_out;  // takes the output's place in the checks of pointers and alignment
+  if (q.out.stride_n < q.Dv) q.out.stride_n = q.Dv;  // (read only: rows may repeat)
+  int rc = validate(&q, true);
+  if (rc != MA_B200_OK) return rc;
+  ma::Geometry g = make_geometry(&q);
+  g.out.sn = gr->grad_out.stride_n;
+  const char* why = "";
+  if (!ma::backward_supported(g, p->qk_dtype, p->v_dtype, &why))
+    return fail(MA_B200_UNSUPPORTED, std::string("backward kernels cannot run this problem: ") + why);
+  const size_t need = ma::backward_layout(g, p->qk_dtype).total;
+  if (workspace == nullptr || reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
+    return fail(MA_B200_INVALID_ARGUMENT, "workspace is NULL or not 256-byte aligned");
+  if (workspace_bytes < need)
+    return fail(MA_B200_WORKSPACE_TOO_SMALL, "workspace has " + std::to_string(workspace_bytes) + " bytes, need " + std::to_string(need));
+  const ma_b200_tensor* outs[3] = {&gr->dq, &gr->dk, &gr->dv};
+  const size_t es = dtype_size(p->qk_dtype), per = 16 / es;
+  ma::View4 v[3];
+  for (int i = 0; i < 3; ++i) {
+    const ma_b200_tensor& t = *outs[i];
+    v[i].ptr = t.ptr; v[i].se = t.stride_e; v[i].sh = t.stride_h; v[i].sn = t.stride_n;
+    if (t.ptr == nullptr) continue;
+    if (reinterpret_cast<uintptr_t>(t.ptr) % 16 != 0 || t.stride_n % per != 0 || t.stride_h % per != 0 || t.stride_e % per != 0 ||
+        t.stride_e < 0 || t.stride_h < 0 || (t.stride_n < p->D && p->N > 1))
+      return fail(MA_B200_INVALID_ARGUMENT, "dq, dk, dv: rows must not overlap and must start on 16-byte boundaries");
+  }
+  const cudaError_t ce = ma::launch_backward(g, p->qk_dtype, g.out, v[0], v[1], v[2], workspace, reinterpret_cast<cudaStream_t>(stream));
+  if (ce != cudaSuccess) return fail(MA_B200_CUDA_ERROR, std::string("backward pass: ") + cudaGetErrorString(ce));
+  return MA_B200_OK;
+}
+
 int ma_b200_device_status(void* workspace, void* stream) {
   if (workspace == nullptr) return fail(MA_B200_INVALID_ARGUMENT, "workspace is NULL");
   int flag = 0;

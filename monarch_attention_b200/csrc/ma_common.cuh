@@ -82,6 +82,16 @@ cudaError_t launch_warp_stage(const Geometry& g, int qk_dtype, StageKind kind, b
 bool head_fused_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
 cudaError_t launch_head_fused(const Geometry& g, int qk_dtype, cudaStream_t stream);
 
+// Backward pass (ma_backward.cu): byte offsets in its workspace; al, ar, cl, cr hold one entry per iteration.
+struct BackwardLayout {
+  size_t mat, vec;  // bytes of one (EH, M*B, D) tensor / (EH, M*B) vector
+  size_t al, ar, cl, cr, y, dal, dy, dar, dcl, dcr, dq_acc, dk_acc, total;
+};
+bool backward_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
+BackwardLayout backward_layout(const Geometry& g, int qk_dtype);
+cudaError_t launch_backward(const Geometry& g, int dtype, const View4& dz, const View4& dq, const View4& dk, const View4& dv,
+                            void* workspace, cudaStream_t stream);
+
 // Tensor-core (tcgen05) path.
 bool tc_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
 // The TMA tensor maps of one call.  tc_plan_get copies them into *plan, from a cache when the same

@@ -264,5 +264,172 @@ struct Tile<float> {
   }
 };
 
+constexpr float kWLog2e = 1.4426950408889634f;
+constexpr float kWLn2 = 0.6931471805599453f;
+
+__device__ __forceinline__ float fast_ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// exp(t) for t <= 0: the 16-bit pipelines round the result to 8 or 11 bits right after, fp32 takes the
+// full-precision function.
+template <typename T>
+__device__ __forceinline__ float exp_of(float t) { return fast_ex2(t * kWLog2e); }
+template <>
+__device__ __forceinline__ float exp_of<float>(float t) { return expf(t); }
+template <typename T>
+__device__ __forceinline__ float log_of(float x) { return __logf(x); }
+template <>
+__device__ __forceinline__ float log_of<float>(float x) { return logf(x); }
+
+// S[16 x KP] (fp32 fragments) = A[16 x DP] * Bt[KP x DP]^T for one warp.  sA points at the warp's first
+// row; both tiles are row-major with pitch PITCH elements.
+template <typename T, int KP, int DP, int PITCH>
+__device__ __forceinline__ void warp_gemm_abt(float (&s)[KP / 8][4], const T* sA, const T* sB, int lane) {
+#pragma unroll
+  for (int nt = 0; nt < KP / 8; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+#pragma unroll
+  for (int kk = 0; kk < DP / 16; ++kk) {
+    typename Tile<T>::A a;
+    Tile<T>::load_a(a, sA + kk * 16, PITCH, lane);
+#pragma unroll
+    for (int np = 0; np < KP / 16; ++np) {
+      typename Tile<T>::B b;
+      Tile<T>::load_b_nk(b, sB + np * 16 * PITCH + kk * 16, PITCH, lane);
+      Tile<T>::mma(s[2 * np], s[2 * np + 1], a, b);
+    }
+  }
+}
+
+// A softmax factor (accumulator fragments of a 16 x KP tile) kept for the contractions that consume it:
+// 16-bit types as packed A fragments, fp32 as it is (the split into two tf32 parts is redone per use).
+template <typename T, int KP>
+struct Factor {
+  typename Tile<T>::A p[KP / 16];
+  __device__ __forceinline__ void set(const float (&s)[KP / 8][4]) {
+#pragma unroll
+    for (int kt = 0; kt < KP / 16; ++kt) Tile<T>::from_acc(p[kt], s[2 * kt], s[2 * kt + 1]);
+  }
+  __device__ __forceinline__ const typename Tile<T>::A& get(int kt) const { return p[kt]; }
+};
+template <int KP>
+struct Factor<float, KP> {
+  float s[KP / 8][4];
+  __device__ __forceinline__ void set(const float (&x)[KP / 8][4]) {
+#pragma unroll
+    for (int nt = 0; nt < KP / 8; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[nt][i] = x[nt][i];
+  }
+  __device__ __forceinline__ Tile<float>::A get(int kt) const {
+    Tile<float>::A a;
+    Tile<float>::from_acc(a, s[2 * kt], s[2 * kt + 1]);
+    return a;
+  }
+};
+
+// O[16 x DP] = P[16 x KP] * V[KP x DP], V row-major.
+template <typename T, int KP, int DP, int PITCH>
+__device__ __forceinline__ void warp_gemm_pv(float (&o)[DP / 8][4], const Factor<T, KP>& p, const T* sV, int lane) {
+#pragma unroll
+  for (int nt = 0; nt < DP / 8; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
+#pragma unroll
+  for (int kt = 0; kt < KP / 16; ++kt) {
+    const typename Tile<T>::A a = p.get(kt);
+#pragma unroll
+    for (int np = 0; np < DP / 16; ++np) {
+      typename Tile<T>::B b;
+      Tile<T>::load_b_kn(b, sV + kt * 16 * PITCH + np * 16, PITCH, lane);
+      Tile<T>::mma(o[2 * np], o[2 * np + 1], a, b);
+    }
+  }
+}
+
+// Writes a warp's 16 x D accumulator tile to global rows: fragments go to a 16-row staging area in
+// shared memory (the warp's own, no longer needed operand rows), then every lane copies 16-byte
+// pieces, so that each 128-byte row is written by eight consecutive lanes.  row_ptr(r) gives the
+// destination of row r (0..15) or nullptr to skip it.
+template <typename T, int DP, int PITCH, typename RowFn>
+__device__ __forceinline__ void store_rows(const float (&o)[DP / 8][4], T* stage, RowFn row_ptr, int D, int lane,
+                                           float post_scale, bool double_round) {
+  const int gq = lane >> 2, t = lane & 3;
+  // The reference rounds the product to storage before scaling it (ma/ma_torch.py:21).  Scaling by a power
+  // of two (1/sqrt(D) for D = 16, 64, 256) commutes with rounding, so one rounding gives the same bits.
+  const bool two_roundings = double_round && (__float_as_uint(post_scale) & 0x007fffffu) != 0u;
+  __syncwarp();
+#pragma unroll
+  for (int nt = 0; nt < DP / 8; ++nt) {
+    const int c = nt * 8 + 2 * t;
+    float v0 = o[nt][0], v1 = o[nt][1], v2 = o[nt][2], v3 = o[nt][3];
+    if (two_roundings) {
+      v0 = round_through<T>(v0); v1 = round_through<T>(v1); v2 = round_through<T>(v2); v3 = round_through<T>(v3);
+    }
+    Tile<T>::store_pair(stage + gq * PITCH + c, v0 * post_scale, v1 * post_scale);
+    Tile<T>::store_pair(stage + (gq + 8) * PITCH + c, v2 * post_scale, v3 * post_scale);
+  }
+  __syncwarp();
+  constexpr int kPer = 16 / (int)sizeof(T), chunks = DP / kPer;  // compile-time, so the row / column split below is shifts
+#pragma unroll
+  for (int i0 = 0; i0 < 16 * chunks; i0 += 32) {
+    const int i = i0 + lane;
+    const int r = i / chunks, c = (i - r * chunks) * kPer;
+    T* dst = (i < 16 * chunks && c < D) ? row_ptr(r) : nullptr;
+    if (dst != nullptr) *reinterpret_cast<uint4*>(dst + c) = *reinterpret_cast<const uint4*>(stage + r * PITCH + c);
+  }
+}
+
+template <typename T>
+constexpr int kF = (int)(sizeof(float) / sizeof(T));  // elements of T in a float
+template <typename T, int DP>
+struct RowPieces { static constexpr int n = DP * (int)sizeof(T) / 16; };
+
+// Row softmax of the logits s[l, m] = round(<q, al>) - cl[m] held as accumulator fragments.
+template <typename T, int KP>
+__device__ __forceinline__ void column_softmax_tail(float (&s)[KP / 8][4], const float* nbias, int lane) {
+  const int t = lane & 3;
+  float mx_lo = -INFINITY, mx_hi = -INFINITY;
+#pragma unroll
+  for (int nt = 0; nt < KP / 8; ++nt) {
+    const float2 bb = *reinterpret_cast<const float2*>(nbias + nt * 8 + 2 * t);  // 8-byte aligned: 2t is even
+    const float b0 = bb.x, b1 = bb.y;  // -cl[m], or -inf beyond M
+    s[nt][0] = round_through<T>(s[nt][0]) + b0;
+    s[nt][1] = round_through<T>(s[nt][1]) + b1;
+    s[nt][2] = round_through<T>(s[nt][2]) + b0;
+    s[nt][3] = round_through<T>(s[nt][3]) + b1;
+    mx_lo = fmaxf(mx_lo, fmaxf(s[nt][0], s[nt][1]));
+    mx_hi = fmaxf(mx_hi, fmaxf(s[nt][2], s[nt][3]));
+  }
+  mx_lo = quad_max(mx_lo);
+  mx_hi = quad_max(mx_hi);
+  float sum_lo = 0.f, sum_hi = 0.f;
+#pragma unroll
+  for (int nt = 0; nt < KP / 8; ++nt) {
+    s[nt][0] = exp_of<T>(s[nt][0] - mx_lo);
+    s[nt][1] = exp_of<T>(s[nt][1] - mx_lo);
+    s[nt][2] = exp_of<T>(s[nt][2] - mx_hi);
+    s[nt][3] = exp_of<T>(s[nt][3] - mx_hi);
+    sum_lo += s[nt][0] + s[nt][1];
+    sum_hi += s[nt][2] + s[nt][3];
+  }
+  const float inv_lo = 1.0f / quad_sum(sum_lo), inv_hi = 1.0f / quad_sum(sum_hi);
+#pragma unroll
+  for (int nt = 0; nt < KP / 8; ++nt) {
+    s[nt][0] *= inv_lo; s[nt][1] *= inv_lo; s[nt][2] *= inv_hi; s[nt][3] *= inv_hi;
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------
+// Logits of the left-factor and output stages for one warp: rows l of column j against all m,
+// w[l,m] = <q[l,j], al[j,m]> - cl[j,m], softmax over m.  Returns the normalised probabilities in s.
+// ---------------------------------------------------------------------------------------------------
+template <typename T, int KP, int DP, int PITCH>
+__device__ __forceinline__ void column_softmax(float (&s)[KP / 8][4], const T* sQw, const T* sAL, const float* nbias,
+                                               int lane) {
+  warp_gemm_abt<T, KP, DP, PITCH>(s, sQw, sAL, lane);
+  column_softmax_tail<T, KP>(s, nbias, lane);
+}
+
 }  // namespace
 }  // namespace ma
