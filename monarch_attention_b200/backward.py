@@ -2,8 +2,8 @@
 
 The reference trains through autograd of its eager implementation (reference:
 ma/ma_torch.py:10-108; experiments/bart fine-tunes through it).  Here the forward result comes from the library's
-kernels and the gradients from its backward kernels (``ma_b200_backward``), which recompute the stage inputs from
-q, k, v, so nothing but the inputs is kept between the two.
+kernels and the gradients from its backward kernels (``ma_b200_backward``, called by the native binding), which recompute
+the stage inputs from q, k, v, so nothing but the inputs is kept between the two.  This module is for the rest.
 
 Problems the backward kernels do not take (block size or block count above 128, fp32 above 64, value width other than
 the key width, widths that are no multiple of 8 or above 80) are differentiated by recomputing the forward ON THE SAME
@@ -15,7 +15,6 @@ Nothing here runs unless an input requires a gradient.
 """
 from __future__ import annotations
 
-import ctypes as C
 import math
 
 import torch
@@ -95,32 +94,8 @@ def differentiable_forward(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tensor | 
     return z[..., gap:, :] if pre_pad else z[..., :N, :]
 
 
-def _kernel_backward(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tensor | None, T: int, B: int, pre_pad: bool,
-                     grad_out: Tensor, needs) -> list[Tensor | None] | None:
-    """Gradients from the backward kernels, or None when they do not take the problem."""
-    from . import _cabi
-    from .monarch_attention import _mask_bytes, _tensor4, _unit_inner, _workspace, make_problem
-    lib = _cabi.load()
-    q, k, v = _unit_inner(q), _unit_inner(k), _unit_inner(v)
-    grad_out = _unit_inner(grad_out.to(v.dtype))
-    if any(s % (16 // grad_out.element_size()) for s in grad_out.stride()[:3]) or grad_out.data_ptr() % 16:
-        grad_out = grad_out.contiguous()
-    mask = _mask_bytes(attn_mask, q.device)
-    prob = make_problem(q, k, v, grad_out, mask, T, B, pre_pad)
-    with torch.cuda.device(q.device):
-        need = lib.ma_b200_backward_workspace_bytes(C.byref(prob))
-        if need == 0:
-            return None
-        grads = [torch.empty_like(t) if want else None for t, want in zip((q, k, v), needs)]
-        gr = _cabi.Gradients(_tensor4(grad_out), *(_tensor4(t) if t is not None else _cabi.Tensor4() for t in grads))
-        stream = torch.cuda.current_stream(q.device).cuda_stream
-        ws = _workspace(q.device, stream, need)
-        _cabi.raise_for_status(lib.ma_b200_backward(C.byref(prob), C.byref(gr), ws.data_ptr(), ws.numel(), stream))
-    return grads
-
-
 class MonarchAttentionFunction(torch.autograd.Function):
-    """forward: the library's kernels; backward: its backward kernels, or autograd through ``differentiable_forward``."""
+    """forward: the library's kernels; backward: autograd through ``differentiable_forward``."""
 
     @staticmethod
     def forward(ctx, q, k, v, attn_mask, T, B, pre_pad, run_kernels):
@@ -132,12 +107,9 @@ class MonarchAttentionFunction(torch.autograd.Function):
     def backward(ctx, grad_out):
         q, k, v = ctx.saved_tensors
         needs = ctx.needs_input_grad[:3]
-        grads = _kernel_backward(q, k, v, ctx.attn_mask, ctx.T, ctx.B, ctx.pre_pad, grad_out, needs)
-        if grads is None:
-            with torch.enable_grad():
-                leaves = [t.detach().requires_grad_(need) for t, need in zip((q, k, v), needs)]
-                z = differentiable_forward(*leaves, ctx.attn_mask, ctx.T, ctx.B, ctx.pre_pad)
-                wanted = [t for t, need in zip(leaves, needs) if need]
-                some = iter(torch.autograd.grad(z, wanted, grad_out.to(z.dtype)))
-            grads = [next(some) if need else None for need in needs]
-        return tuple(grads) + (None,) * 5
+        with torch.enable_grad():
+            leaves = [t.detach().requires_grad_(need) for t, need in zip((q, k, v), needs)]
+            z = differentiable_forward(*leaves, ctx.attn_mask, ctx.T, ctx.B, ctx.pre_pad)
+            wanted = [t for t, need in zip(leaves, needs) if need]
+            grads = iter(torch.autograd.grad(z, wanted, grad_out.to(z.dtype)))
+        return tuple(next(grads) if need else None for need in needs) + (None,) * 5

@@ -1,8 +1,8 @@
-"""Build the C-ABI shared library (sm_100a only) in-tree with nvcc.
+"""Build the C-ABI shared library (sm_100a only) in-tree with nvcc, and the Python binding on top of it.
 
     python -m monarch_attention_b200.build [--force] [--verbose]
 
-Output: monarch_attention_b200/lib/libmonarch_attention_b200.so
+Output: monarch_attention_b200/lib/libmonarch_attention_b200.so and monarch_attention_b200/_native.so
 """
 from __future__ import annotations
 
@@ -11,11 +11,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libmonarch_attention_b200.so")
+NATIVE_PATH = os.path.join(PKG, "_native.so")
+NATIVE_SOURCE = "ma_torch.cpp"
 SOURCES = ["ma_api.cu", "ma_generic.cu", "ma_tc.cu", "ma_fused.cu", "ma_warp.cu", "ma_backward.cu", "ma_noalloc.cu", "ma_host.cu"]
 HEADERS = ["ma_common.cuh", "ma_warp_common.cuh", "ma_warp_kernels.inc", "ma_warp_wide.inc", "ma_warp_head.inc", "ma_sm100.cuh", "ma_tc_plan.cuh", os.path.join("..", "..", "include", "monarch_attention_b200.h")]
 
@@ -34,39 +37,55 @@ def find_nvcc() -> str:
     raise RuntimeError("nvcc not found (set NVCC=/path/to/nvcc)")
 
 
-def is_stale() -> bool:
-    if not os.path.exists(LIB_PATH):
-        return True
-    built = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, s) for s in SOURCES + HEADERS] + [os.path.abspath(__file__)]
-    return any(os.path.getmtime(d) > built for d in deps)
+def _newest(names) -> float:
+    return max(os.path.getmtime(os.path.join(CSRC, n)) for n in names)
+
+
+def _older(path: str, than: float) -> bool:
+    return not os.path.exists(path) or os.path.getmtime(path) < than
+
+
+def _native_command(obj: str) -> list[str]:
+    from torch.utils.cpp_extension import include_paths
+    inc = [f"-I{p}" for p in include_paths() + ["/usr/local/cuda/include", sysconfig.get_paths()["include"]]]
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-DTORCH_API_INCLUDE_EXTENSION_H",
+            "-DTORCH_EXTENSION_NAME=_native", *inc, "-c", os.path.join(CSRC, NATIVE_SOURCE), "-o", obj]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not is_stale():
-        return LIB_PATH
-    nvcc = find_nvcc()
+    """Compiles what is older than its sources: the headers count for every source."""
     os.makedirs(LIB_DIR, exist_ok=True)
-    objs = []
-    procs = []
-    for src in SOURCES:
-        obj = os.path.join(LIB_DIR, src.replace(".cu", ".o"))
-        cmd = [nvcc, *NVCC_FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
-        if verbose:
-            cmd[1:1] = ["-Xptxas", "-v"]
-        procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
-        objs.append(obj)
+    common = max(_newest(HEADERS), os.path.getmtime(os.path.abspath(__file__)))
+    jobs, objs = [], []
+    for src in [NATIVE_SOURCE] + SOURCES:
+        obj = os.path.join(LIB_DIR, os.path.splitext(src)[0] + ".o")
+        if src != NATIVE_SOURCE:
+            objs.append(obj)
+        if not force and not _older(obj, max(common, _newest([src]))):
+            continue
+        if src == NATIVE_SOURCE:
+            cmd = _native_command(obj)
+        else:
+            cmd = [find_nvcc(), *(["-Xptxas", "-v"] if verbose else []), *NVCC_FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
+        jobs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     failed = False
-    for src, p in procs:
+    for src, p in jobs:
         out, _ = p.communicate()
         if p.returncode != 0 or verbose:
-            print(f"--- nvcc {src} ---\n{out}", file=sys.stderr)
+            print(f"--- {src} ---\n{out}", file=sys.stderr)
         failed |= p.returncode != 0
     if failed:
-        raise RuntimeError("nvcc failed")
-    link = [nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC",
-            "-o", LIB_PATH, *objs, "-cudart", "static"]
-    subprocess.check_call(link)
+        raise RuntimeError("compilation failed")
+    newest = max(os.path.getmtime(o) for o in objs)
+    if _older(LIB_PATH, newest):
+        subprocess.check_call([find_nvcc(), "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC",
+                               "-o", LIB_PATH, *objs, "-cudart", "static"])
+    native_obj = os.path.join(LIB_DIR, os.path.splitext(NATIVE_SOURCE)[0] + ".o")
+    if _older(NATIVE_PATH, os.path.getmtime(native_obj)):
+        from torch.utils.cpp_extension import library_paths
+        subprocess.check_call(["g++", "-shared", "-o", NATIVE_PATH, native_obj, f"-L{LIB_DIR}", "-l:" + os.path.basename(LIB_PATH),
+                               "-Wl,-rpath,$ORIGIN/lib", *(f"-L{p}" for p in library_paths()), "-lc10", "-lc10_cuda",
+                               "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"])
     return LIB_PATH
 
 

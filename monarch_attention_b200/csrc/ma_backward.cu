@@ -476,10 +476,7 @@ cudaError_t backward_launch(const BackwardArgs& a, BackwardStage st, size_t* sme
     case kBackRight: fn = (const void*)backward_right_kernel<T, KP, DP, false>; break;
     case kBackRightWithV: fn = (const void*)backward_right_kernel<T, KP, DP, true>; break;
   }
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  if (const cudaError_t e = allow_dynamic_smem(fn, smem); e != cudaSuccess) return e;
   const int rows = right ? g.B : g.M;
   void* args[] = {(void*)&a};
   return cudaLaunchKernel(fn, dim3(right ? g.M : g.B, g.E * g.H), dim3(2 * ((rows + 15) & ~15)), args, smem, stream);

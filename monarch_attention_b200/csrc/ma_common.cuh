@@ -6,6 +6,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <map>
+#include <mutex>
+#include <utility>
+
 #include "../../include/monarch_attention_b200.h"
 
 namespace ma {
@@ -63,6 +67,23 @@ struct Cvt<__half> {
 template <typename T>
 __device__ __forceinline__ float round_through(float x) {
   return Cvt<T>::to_f(Cvt<T>::from_f(x));
+}
+
+// Lets `fn` use up to `bytes` of dynamic shared memory on the current device.  The runtime call takes longer than
+// queuing a launch, so it is made only when a larger size than before is asked for.
+inline cudaError_t allow_dynamic_smem(const void* fn, size_t bytes) {
+  if (bytes <= 48 * 1024) return cudaSuccess;
+  static std::mutex mutex;
+  static std::map<std::pair<int, const void*>, size_t> allowed;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mutex);
+  size_t& have = allowed[{dev, fn}];
+  if (bytes <= have) return cudaSuccess;
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) have = bytes;
+  return e;
 }
 
 // Host-side launchers implemented by the kernel translation units.

@@ -574,8 +574,7 @@ cudaError_t launch_typed(const Geometry& g, StageKind kind, bool first, cudaStre
   const dim3 block(kThreads);
   const int EH = g.E * g.H;
   auto raise = [&](const void* fn) -> cudaError_t {
-    if (smem > 48 * 1024) return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return cudaSuccess;
+    return allow_dynamic_smem(fn, smem);
   };
   cudaError_t err = cudaSuccess;
   if (small_tiles(g)) {

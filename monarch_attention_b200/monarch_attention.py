@@ -13,7 +13,6 @@ path here.
 """
 from __future__ import annotations
 
-import ctypes as C
 from collections.abc import Callable
 from enum import StrEnum
 
@@ -36,28 +35,8 @@ class PadType(StrEnum):
     post = "post"
 
 
-# ---------------------------------------------------------------------------------
-# Workspace cache: one scratch tensor per (device, stream), grown on demand.  It comes
-# from PyTorch's caching allocator, so steady-state calls allocate nothing.
-# ---------------------------------------------------------------------------------
-_workspaces: dict[tuple[int, int], Tensor] = {}
-
-
-def _workspace(device: torch.device, stream: int, nbytes: int) -> Tensor:
-    key = (device.index if device.index is not None else torch.cuda.current_device(), stream)
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
-
-
 def _tensor4(t: Tensor) -> _cabi.Tensor4:
     return _cabi.Tensor4(t.data_ptr(), t.stride(0), t.stride(1), t.stride(2))
-
-
-def _unit_inner(t: Tensor) -> Tensor:
-    return t if t.stride(-1) == 1 or t.shape[-1] == 1 else t.contiguous()
 
 
 def make_problem(q: Tensor, k: Tensor, v: Tensor, out: Tensor, mask: Tensor | None, T: int, B: int, pre_pad: bool,
@@ -77,18 +56,8 @@ def make_problem(q: Tensor, k: Tensor, v: Tensor, out: Tensor, mask: Tensor | No
     return p
 
 
-def _check_inputs(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tensor | None):
-    if q.dim() != 4 or k.dim() != 4 or v.dim() != 4:
-        raise ValueError("query, key and value must have shape (batch, heads, tokens, width)")
-    if not q.is_cuda:
-        raise RuntimeError("monarch_attention_b200 runs on CUDA tensors only (there is no CPU path)")
-    if k.device != q.device or v.device != q.device:
-        raise ValueError("query, key and value must be on the same device")
-    _check_device_free_inputs(q, k, v, attn_mask)
-
-
 def _check_device_free_inputs(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tensor | None):
-    """Shape and dtype rules shared by the device and the host entry points."""
+    """Shape and dtype rules of the host entry point (those of the device entry point are in the native binding)."""
     if q.dim() != 4 or k.dim() != 4 or v.dim() != 4:
         raise ValueError("query, key and value must have shape (batch, heads, tokens, width)")
     if k.shape != q.shape:
@@ -103,13 +72,20 @@ def _check_device_free_inputs(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tensor
         raise ValueError(f"attention_mask must have shape (batch, tokens) = {(q.shape[0], q.shape[2])}")
 
 
-def _mask_bytes(attn_mask: Tensor | None, device) -> Tensor | None:
-    """Any-dtype mask (non-zero = valid; reference: ma/ma_torch.py:96-98) -> uint8, unit inner stride."""
-    if attn_mask is None:
-        return None
-    m = attn_mask.to(device)
-    m = m.view(torch.uint8) if m.dtype == torch.bool else (m != 0).view(torch.uint8)
-    return m if m.stride(-1) == 1 else m.contiguous()
+_native_forward = None
+
+
+def _load_native():
+    """The native entry point (monarch_attention_b200/_native.so); raises RuntimeError when it has not been built."""
+    global _native_forward
+    _cabi.load()
+    try:
+        from . import _native
+    except ImportError as err:
+        raise RuntimeError("monarch_attention_b200/_native.so is missing or does not match this PyTorch: build it with "
+                           "`python -m monarch_attention_b200.build`. There is no fallback implementation.") from err
+    _native_forward = _native.forward
+    return _native_forward
 
 
 def monarch_attention_b200(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tensor | None, T: int, B: int, pre_pad: bool,
@@ -123,39 +99,14 @@ def monarch_attention_b200(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tensor | 
     in the layout the model adapters produce with ``permute(0, 2, 1, 3).contiguous()`` after the call
     (reference: experiments/vit/model.py:99-101), which then costs nothing.
     """
-    _check_inputs(q, k, v, attn_mask)
-    if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
-        # training: the kernels give the result, the gradients come from recomputation (backward.py)
-        if out is not None:
-            raise ValueError("out= cannot be combined with inputs that require a gradient")
+    fn = _native_forward or _load_native()
+    result = fn(q, k, v, attn_mask, T, B, pre_pad, kernel, out, token_major_output)
+    if result is None:   # a gradient is wanted that the backward kernels do not give
         from .backward import MonarchAttentionFunction
-        return MonarchAttentionFunction.apply(
+        result = MonarchAttentionFunction.apply(
             q, k, v, attn_mask, T, B, pre_pad,
-            lambda a, b, c: monarch_attention_b200(a, b, c, attn_mask, T, B, pre_pad, kernel=kernel,
-                                                   token_major_output=token_major_output))
-    lib = _cabi.load()
-    dev_index = q.device.index if q.device.index is not None else torch.cuda.current_device()
-    # A bounded wait of an earlier asynchronous call on this device that gave up is reported here, at the
-    # next call, without a synchronisation (the kernel leaves its code in mapped host memory).
-    _cabi.raise_for_status(lib.ma_b200_poll_device_status(dev_index))
-    q, k, v = _unit_inner(q), _unit_inner(k), _unit_inner(v)
-    E, H, N, _ = q.shape
-    if out is None:
-        if token_major_output:
-            out = torch.empty((E, N, H, v.shape[-1]), dtype=v.dtype, device=v.device).permute(0, 2, 1, 3)
-        else:
-            out = torch.empty((E, H, N, v.shape[-1]), dtype=v.dtype, device=v.device)
-    mask = _mask_bytes(attn_mask, q.device)
-    prob = make_problem(q, k, v, out, mask, T, B, pre_pad, kernel)
-    with torch.cuda.device(q.device):
-        need = lib.ma_b200_workspace_bytes(C.byref(prob))
-        if need == 0:
-            _cabi.raise_for_status(lib.ma_b200_workspace_layout_of(C.byref(prob), C.byref(_cabi.WorkspaceLayout())))
-        stream = torch.cuda.current_stream(q.device).cuda_stream
-        ws = _workspace(q.device, stream, need)
-        rc = lib.ma_b200_forward(C.byref(prob), ws.data_ptr(), ws.numel(), stream)
-    _cabi.raise_for_status(rc)
-    return out
+            lambda a, b, c: fn(a, b, c, attn_mask, T, B, pre_pad, kernel, None, token_major_output))
+    return result
 
 
 def _generic(q, k, v, m, T, B, pre_pad):
