@@ -42,7 +42,7 @@ int validate(const ma_b200_problem* p, bool need_pointers) {
     return fail(MA_B200_INVALID_ARGUMENT, "unknown dtype");
   if (!(p->qk_dtype == p->v_dtype || p->v_dtype == MA_B200_F32))
     return fail(MA_B200_UNSUPPORTED, "v_dtype must equal qk_dtype or be f32");
-  if (p->kernel < MA_B200_KERNEL_AUTO || p->kernel > MA_B200_KERNEL_TF32X3 || p->kernel == 4)
+  if (p->kernel < MA_B200_KERNEL_AUTO || p->kernel > MA_B200_KERNEL_HEAD_RESIDENT || p->kernel == 4)
     return fail(MA_B200_INVALID_ARGUMENT, "unknown kernel family");
   if ((long long)p->E * p->H > 0x7fffffffLL / 2) return fail(MA_B200_INVALID_ARGUMENT, "E*H too large");
   if (need_pointers) {
@@ -98,6 +98,10 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, int* kernel)
   const bool head_ok = ma::head_fused_supported(g, p->qk_dtype, p->v_dtype, &why_h);
   if (p->kernel == MA_B200_KERNEL_HEAD_FUSED && !head_ok)
     return fail(MA_B200_UNSUPPORTED, std::string("one-CTA-per-head kernel cannot run this problem: ") + why_h);
+  const char* why_r = "";
+  const bool resident_ok = ma::head_resident_supported(g, p->qk_dtype, p->v_dtype, &why_r);
+  if (p->kernel == MA_B200_KERNEL_HEAD_RESIDENT && !resident_ok)
+    return fail(MA_B200_UNSUPPORTED, std::string("head-resident kernel cannot run this problem: ") + why_r);
   const char* why_x = "";
   const bool tf32_ok = ma::tf32x3_supported(g, p->qk_dtype, p->v_dtype, &why_x);
   if (p->kernel == MA_B200_KERNEL_TF32X3 && !tf32_ok)
@@ -108,7 +112,7 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, int* kernel)
   if (p->kernel == MA_B200_KERNEL_AUTO)
     // (the one-CTA-per-head kernel is selectable but not preferred: on the ViT / RoBERTa shapes it
     // measured slower than the two staged launches - these tiny tiles are instruction-bound)
-    *kernel = tc_ok ? MA_B200_KERNEL_TCGEN05 : (warp_ok ? MA_B200_KERNEL_WARP_MMA : (tf32_pays ? MA_B200_KERNEL_TF32X3 : MA_B200_KERNEL_GENERIC));
+    *kernel = tc_ok ? MA_B200_KERNEL_TCGEN05 : resident_ok ? MA_B200_KERNEL_HEAD_RESIDENT : (warp_ok ? MA_B200_KERNEL_WARP_MMA : (tf32_pays ? MA_B200_KERNEL_TF32X3 : MA_B200_KERNEL_GENERIC));
   else *kernel = p->kernel;
   if (*kernel == MA_B200_KERNEL_GENERIC) {
     const size_t need = ma::generic_stage_smem_bytes(g, g.B > g.M ? ma::kStageRight : ma::kStageLeft);
@@ -172,7 +176,7 @@ int run_forward(const ma_b200_problem* p, void* workspace, size_t workspace_byte
   // Status word and stage-completion counters start at zero.  The stage kernels that wait for nothing clear the
   // status word themselves: a memset in front of them is 1.5 us on the stream, as much as a small kernel.
   cudaError_t ce = cudaSuccess;
-  if (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3) {
+  if (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3 && L.kernel != MA_B200_KERNEL_HEAD_RESIDENT) {
     ce = cudaMemsetAsync(ws + L.status, 0, L.ar - L.status, stream);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(status, counters)");
   }
@@ -209,8 +213,9 @@ int run_forward(const ma_b200_problem* p, void* workspace, size_t workspace_byte
 
   rc = MA_B200_OK;
   bool first = true;
-  if (L.kernel == MA_B200_KERNEL_HEAD_FUSED) {
-    ce = ma::launch_head_fused(g, p->qk_dtype, stream);
+  if (L.kernel == MA_B200_KERNEL_HEAD_FUSED || L.kernel == MA_B200_KERNEL_HEAD_RESIDENT) {
+    ce = L.kernel == MA_B200_KERNEL_HEAD_FUSED ? ma::launch_head_fused(g, p->qk_dtype, stream)
+                                               : ma::launch_head_resident(g, p->qk_dtype, stream);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "one-CTA-per-head kernel");
     if (ev != nullptr)
       for (int i = 1; i <= n_stages; ++i) cudaEventRecord(ev[i], stream);

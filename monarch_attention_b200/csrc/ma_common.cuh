@@ -113,6 +113,10 @@ BackwardLayout backward_layout(const Geometry& g, int qk_dtype);
 cudaError_t launch_backward(const Geometry& g, int dtype, const View4& dz, const View4& dq, const View4& dk, const View4& dv,
                             void* workspace, cudaStream_t stream);
 
+// Head-resident kernel: all stages of a head in one launch, block size and count up to 32 (ma_head.cu).
+bool head_resident_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
+cudaError_t launch_head_resident(const Geometry& g, int qk_dtype, cudaStream_t stream);
+
 // Tensor-core (tcgen05) path.
 bool tc_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
 // The TMA tensor maps of one call.  tc_plan_get copies them into *plan, from a cache when the same

@@ -66,6 +66,32 @@ __device__ __forceinline__ float quad_sum(float v) {
   return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
+// Sums over the eight lanes lane/4 of N values per lane (N a power of two, at least 4), by halving: a step sends one
+// half of the values to the partner and keeps the other, so N values take about N shuffles instead of 3 N.  Returns
+// the index of the first of the values left in this lane; N/8 values are left (one, twice over, when N = 4).
+template <int N>
+__device__ __forceinline__ int reduce_rows(float (&v)[N], int lane) {
+  int base = 0;
+  int n = N;
+#pragma unroll
+  for (int d = 16; d >= 4; d >>= 1) {
+    if (n > 1) {
+      const bool up = (lane & d) != 0;
+      n >>= 1;
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i)
+        if (i < n) {
+          const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+        }
+      if (up) base += n;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], d);
+    }
+  }
+  return base;
+}
+
 // Copies `rows` rows of `width` elements (a multiple of 8) into a shared tile with row
 // pitch `pitch` elements, zero-filling rows that do not exist, columns past width and rows
 // [rows, rpad).  Threads tid of nthreads cooperate.  The copies are asynchronous (cp.async, 16 bytes
