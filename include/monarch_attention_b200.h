@@ -53,7 +53,7 @@ enum {
 enum { MA_B200_F32 = 0, MA_B200_BF16 = 1, MA_B200_F16 = 2 };
 
 /* Kernel families.  AUTO picks the fused tcgen05 kernel when the problem fits it, else the
- * head-resident kernel, else the warp-level tensor-core kernels (16-bit or fp32), else the generic kernels.
+ * head-resident kernel, else the tcgen05 tile kernels, else the warp-level tensor-core kernels (16-bit or fp32), else the generic kernels.
  *   GENERIC        SIMT stage kernels, any shape / dtype / mask (2T launches)
  *   TCGEN05        persistent tcgen05 kernel, all 2T stages in one launch: 16-bit inputs,
  *                  D = Dv = 64, no mask, no padding, block size = block count = 128 or 64
@@ -67,7 +67,9 @@ enum { MA_B200_F32 = 0, MA_B200_BF16 = 1, MA_B200_F16 = 2 };
  *   TF32X3         the WARP_MMA stage kernels on f32 tensors, block size and block count up to 128,
  *                  D <= 80 (multiple of 8): every operand split into two tf32 parts (2T launches)
  *   HEAD_RESIDENT  16-bit inputs, block size and block count up to 32, D <= 80 (multiple of 8): one CTA
- *                  or cluster per head, all stages in one launch, the head's state on chip where it fits */
+ *                  or cluster per head, all stages in one launch, the head's state on chip where it fits
+ *   TILE           tcgen05 stage kernels, one 128-row tile per CTA: 16-bit inputs, block size and block count
+ *                  up to 256, D <= 64 (multiple of 8), masks and padding (2T launches) */
 enum {
   MA_B200_KERNEL_AUTO = 0,
   MA_B200_KERNEL_GENERIC = 1,
@@ -76,7 +78,8 @@ enum {
   MA_B200_KERNEL_WARP_MMA = 5,
   MA_B200_KERNEL_HEAD_FUSED = 6,
   MA_B200_KERNEL_TF32X3 = 7,
-  MA_B200_KERNEL_HEAD_RESIDENT = 8
+  MA_B200_KERNEL_HEAD_RESIDENT = 8,
+  MA_B200_KERNEL_TILE = 9
 };
 
 typedef struct ma_b200_tensor {

@@ -11,11 +11,12 @@ import os
 ABI_VERSION = 1
 F32, BF16, F16 = 0, 1, 2
 KERNEL_AUTO, KERNEL_GENERIC, KERNEL_TCGEN05, KERNEL_TCGEN05_STAGED, KERNEL_WARP_MMA, KERNEL_HEAD_FUSED = 0, 1, 2, 3, 5, 6
-KERNEL_TF32X3, KERNEL_HEAD_RESIDENT = 7, 8
+KERNEL_TF32X3, KERNEL_HEAD_RESIDENT, KERNEL_TILE = 7, 8, 9
 KERNEL_NAMES = {KERNEL_AUTO: "auto", KERNEL_GENERIC: "generic", KERNEL_TCGEN05: "tcgen05-fused",
                 KERNEL_TCGEN05_STAGED: "tcgen05-staged",
                 KERNEL_WARP_MMA: "warp-mma", KERNEL_HEAD_FUSED: "head-fused",
-                KERNEL_TF32X3: "tf32x3", KERNEL_HEAD_RESIDENT: "head-resident"}
+                KERNEL_TF32X3: "tf32x3", KERNEL_HEAD_RESIDENT: "head-resident",
+                KERNEL_TILE: "tile"}
 OK, INVALID_ARGUMENT, UNSUPPORTED, CUDA_ERROR, DEVICE_WAIT_EXPIRED, WORKSPACE_TOO_SMALL = range(6)
 
 LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libmonarch_attention_b200.so")

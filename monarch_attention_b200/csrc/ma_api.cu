@@ -42,7 +42,7 @@ int validate(const ma_b200_problem* p, bool need_pointers) {
     return fail(MA_B200_INVALID_ARGUMENT, "unknown dtype");
   if (!(p->qk_dtype == p->v_dtype || p->v_dtype == MA_B200_F32))
     return fail(MA_B200_UNSUPPORTED, "v_dtype must equal qk_dtype or be f32");
-  if (p->kernel < MA_B200_KERNEL_AUTO || p->kernel > MA_B200_KERNEL_HEAD_RESIDENT || p->kernel == 4)
+  if (p->kernel < MA_B200_KERNEL_AUTO || p->kernel > MA_B200_KERNEL_TILE || p->kernel == 4)
     return fail(MA_B200_INVALID_ARGUMENT, "unknown kernel family");
   if ((long long)p->E * p->H > 0x7fffffffLL / 2) return fail(MA_B200_INVALID_ARGUMENT, "E*H too large");
   if (need_pointers) {
@@ -102,6 +102,10 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, int* kernel)
   const bool resident_ok = ma::head_resident_supported(g, p->qk_dtype, p->v_dtype, &why_r);
   if (p->kernel == MA_B200_KERNEL_HEAD_RESIDENT && !resident_ok)
     return fail(MA_B200_UNSUPPORTED, std::string("head-resident kernel cannot run this problem: ") + why_r);
+  const char* why_t = "";
+  const bool tile_ok = ma::tile_supported(g, p->qk_dtype, p->v_dtype, &why_t);
+  if (p->kernel == MA_B200_KERNEL_TILE && !tile_ok)
+    return fail(MA_B200_UNSUPPORTED, std::string("tcgen05 tile kernels cannot run this problem: ") + why_t);
   const char* why_x = "";
   const bool tf32_ok = ma::tf32x3_supported(g, p->qk_dtype, p->v_dtype, &why_x);
   if (p->kernel == MA_B200_KERNEL_TF32X3 && !tf32_ok)
@@ -112,7 +116,7 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, int* kernel)
   if (p->kernel == MA_B200_KERNEL_AUTO)
     // (the one-CTA-per-head kernel is selectable but not preferred: on the ViT / RoBERTa shapes it
     // measured slower than the two staged launches - these tiny tiles are instruction-bound)
-    *kernel = tc_ok ? MA_B200_KERNEL_TCGEN05 : resident_ok ? MA_B200_KERNEL_HEAD_RESIDENT : (warp_ok ? MA_B200_KERNEL_WARP_MMA : (tf32_pays ? MA_B200_KERNEL_TF32X3 : MA_B200_KERNEL_GENERIC));
+    *kernel = tc_ok ? MA_B200_KERNEL_TCGEN05 : resident_ok ? MA_B200_KERNEL_HEAD_RESIDENT : tile_ok ? MA_B200_KERNEL_TILE : (warp_ok ? MA_B200_KERNEL_WARP_MMA : (tf32_pays ? MA_B200_KERNEL_TF32X3 : MA_B200_KERNEL_GENERIC));
   else *kernel = p->kernel;
   if (*kernel == MA_B200_KERNEL_GENERIC) {
     const size_t need = ma::generic_stage_smem_bytes(g, g.B > g.M ? ma::kStageRight : ma::kStageLeft);
@@ -176,7 +180,8 @@ int run_forward(const ma_b200_problem* p, void* workspace, size_t workspace_byte
   // Status word and stage-completion counters start at zero.  The stage kernels that wait for nothing clear the
   // status word themselves: a memset in front of them is 1.5 us on the stream, as much as a small kernel.
   cudaError_t ce = cudaSuccess;
-  if (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3 && L.kernel != MA_B200_KERNEL_HEAD_RESIDENT) {
+  if (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3 && L.kernel != MA_B200_KERNEL_HEAD_RESIDENT &&
+      L.kernel != MA_B200_KERNEL_TILE) {
     ce = cudaMemsetAsync(ws + L.status, 0, L.ar - L.status, stream);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(status, counters)");
   }
@@ -191,6 +196,13 @@ int run_forward(const ma_b200_problem* p, void* workspace, size_t workspace_byte
     plan = &plan_store;
   }
 
+  int* host_status = nullptr;
+  if (L.kernel == MA_B200_KERNEL_TILE) {
+    int dev = 0;
+    if ((ce = cudaGetDevice(&dev)) != cudaSuccess) return cuda_fail(ce, "cudaGetDevice");
+    host_status = ma::host_status_word(dev);
+  }
+
   const int n_stages = 2 * p->num_steps;
   cudaEvent_t* ev = nullptr;
   if (stage_ms != nullptr) {
@@ -203,6 +215,8 @@ int run_forward(const ma_b200_problem* p, void* workspace, size_t workspace_byte
     cudaError_t e;
     if (L.kernel == MA_B200_KERNEL_TCGEN05_STAGED)
       e = ma::launch_fused(plan, g, counters, stage_idx, stage_idx + 1, 0, stream);
+    else if (L.kernel == MA_B200_KERNEL_TILE)
+      e = ma::launch_tile_stage(g, p->qk_dtype, kind, first, host_status, stream);
     else if (L.kernel == MA_B200_KERNEL_WARP_MMA || L.kernel == MA_B200_KERNEL_TF32X3)
       e = ma::launch_warp_stage(g, p->qk_dtype, kind, first, stream);
     else e = ma::launch_generic_stage(g, p->qk_dtype, p->v_dtype, kind, first, stream);

@@ -129,6 +129,11 @@ void tc_plan_destroy(TcPlan* plan);
 size_t fused_counter_bytes(const Geometry& g);
 cudaError_t launch_fused(const TcPlan* plan, const Geometry& g, int* counters, int stage_begin, int stage_end,
                          int wait_deps, cudaStream_t stream);
+// Device address of the mapped host word that a kernel whose bounded wait gave up stores its code in (nullptr: none).
+int* host_status_word(int device);
+// tcgen05 stage kernels, one 128-row tile per CTA: block size and count up to 256, D <= 64, masks and padding (ma_tile.cu).
+bool tile_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
+cudaError_t launch_tile_stage(const Geometry& g, int dtype, StageKind kind, bool first, int* host_status, cudaStream_t stream);
 // Code of a bounded device-side wait that gave up on `device` since the last poll (0 = none); reads a mapped
 // host word, so it needs no synchronisation.
 int fused_poll_status(int device);

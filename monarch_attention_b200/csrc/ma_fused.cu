@@ -874,6 +874,28 @@ int fused_poll_status(int device) {
   return code;
 }
 
+int* host_status_word(int device) {
+  if (device < 0 || device >= 64) return nullptr;
+  std::lock_guard<std::mutex> lock(g_host_status_mutex);
+  HostStatus& hs = g_host_status[device];
+  if (!hs.tried) {
+    hs.tried = true;
+    void* hp = nullptr;
+    if (cudaHostAlloc(&hp, 64, cudaHostAllocMapped) == cudaSuccess) {
+      *reinterpret_cast<int*>(hp) = 0;
+      void* dp = nullptr;
+      if (cudaHostGetDevicePointer(&dp, hp, 0) == cudaSuccess) {
+        hs.host = reinterpret_cast<int*>(hp);
+        hs.dev = reinterpret_cast<int*>(dp);
+      } else {
+        cudaFreeHost(hp);
+      }
+    }
+    (void)cudaGetLastError();
+  }
+  return hs.dev;
+}
+
 static int g_spin_limit_override = 0;
 void fused_set_spin_limit(int iterations) { g_spin_limit_override = iterations; }
 
@@ -888,9 +910,8 @@ cudaError_t launch_fused(const TcPlan* plan, const Geometry& g, int* counters, i
   const int variant = (g.B == kTile ? 0 : 2) + (bf ? 0 : 1);
   const void* fn = g.B == kTile ? (bf ? (const void*)fused_kernel<__nv_bfloat16, 1> : (const void*)fused_kernel<__half, 1>)
                                 : (bf ? (const void*)fused_kernel<__nv_bfloat16, 2> : (const void*)fused_kernel<__half, 2>);
-  int* host_status_dev = nullptr;
   {
-    // once per device and kernel variant: shared-memory opt-in, SM count, the mapped status word
+    // once per device and kernel variant: shared-memory opt-in and SM count
     std::lock_guard<std::mutex> lock(g_host_status_mutex);
     if (!g_attr_done[dev][variant]) {
       e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
@@ -906,24 +927,8 @@ cudaError_t launch_fused(const TcPlan* plan, const Geometry& g, int* counters, i
         return cudaErrorLaunchOutOfResources;
       g_attr_done[dev][variant] = true;
     }
-    HostStatus& hs = g_host_status[dev];
-    if (!hs.tried) {
-      hs.tried = true;
-      void* hp = nullptr;
-      if (cudaHostAlloc(&hp, 64, cudaHostAllocMapped) == cudaSuccess) {
-        *reinterpret_cast<int*>(hp) = 0;
-        void* dp = nullptr;
-        if (cudaHostGetDevicePointer(&dp, hp, 0) == cudaSuccess) {
-          hs.host = reinterpret_cast<int*>(hp);
-          hs.dev = reinterpret_cast<int*>(dp);
-        } else {
-          cudaFreeHost(hp);
-        }
-      }
-      (void)cudaGetLastError();
-    }
-    host_status_dev = hs.dev;
   }
+  int* const host_status_dev = host_status_word(dev);
   const int sms = g_sm_count[dev];
   FusedArgs a;
   a.stage_begin = stage_begin;

@@ -138,6 +138,8 @@ register_impl("b200-tf32x3",
               lambda q, k, v, m, T, B, pp: monarch_attention_b200(q, k, v, m, T, B, pp, kernel=_cabi.KERNEL_TF32X3))
 register_impl("b200-head-resident",
               lambda q, k, v, m, T, B, pp: monarch_attention_b200(q, k, v, m, T, B, pp, kernel=_cabi.KERNEL_HEAD_RESIDENT))
+register_impl("b200-tile",
+              lambda q, k, v, m, T, B, pp: monarch_attention_b200(q, k, v, m, T, B, pp, kernel=_cabi.KERNEL_TILE))
 
 
 class MonarchAttention(nn.Module):
@@ -148,7 +150,8 @@ class MonarchAttention(nn.Module):
     launch), "b200-tcgen05-staged" (same kernel, one launch per stage),
     "b200-warp-mma" (warp-level tensor-core kernels for small blocks),
     "b200-head-fused" (one CTA per head, one iteration, state in shared memory), "b200-tf32x3"
-    (the warp-level kernels on fp32 tensors) or "b200-head-resident" (one CTA or cluster per head, all stages).  The reference's
+    (the warp-level kernels on fp32 tensors), "b200-head-resident" (one CTA or cluster per head, all stages) or
+    "b200-tile" (tcgen05 stage kernels, one 128-row tile per CTA).  The reference's
     "torch" and "triton" implementations are not part of this library; asking for an
     unknown name raises ``ValueError`` exactly as the reference does.
     """

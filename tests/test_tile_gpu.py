@@ -1,0 +1,45 @@
+"""tcgen05 tile kernels at the edges of their tiles (two units per tile with an odd last one, row and column remainders,
+the row behind the last whole block, both padding sides, masks that empty blocks, narrow heads, several tiles per CTA),
+against the CPU oracle."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [  # E, H, N, D, B, T, pad, mask
+    (1, 1, 64 * 64, 64, 64, 1, "post", "none"), (1, 2, 64 * 64, 64, 64, 2, "post", "none"),
+    (2, 2, 64 * 61 - 7, 64, 64, 2, "post", "tail"), (1, 3, 45 * 47 - 11, 64, 45, 3, "pre", "rand"),
+    (1, 1, 33 * 64, 64, 33, 2, "post", "none"), (1, 2, 128 * 128, 64, 128, 2, "post", "none"),
+    (1, 1, 65 * 128 - 64, 64, 65, 2, "pre", "none"), (2, 1, 97 * 100 - 3, 64, 97, 2, "post", "block"),
+    (1, 1, 129 * 40, 64, 129, 2, "post", "none"), (1, 1, 40 * 129 - 39, 64, 40, 2, "pre", "rand"),
+    (1, 1, 256 * 256, 64, 256, 2, "post", "none"), (1, 1, 200 * 170 - 100, 64, 200, 1, "pre", "rand"),
+    (1, 2, 60 * 70 - 1, 40, 60, 2, "post", "none"), (1, 2, 70 * 60, 32, 70, 3, "pre", "tail"), (1, 1, 150 * 66 - 20, 8, 150, 2, "post", "none"),
+    (1, 1, 36 * 2 - 1, 64, 36, 2, "post", "none"), (1, 1, 20 * 3, 16, 20, 2, "pre", "none"),
+    (8, 12, 40 * 38 - 3, 64, 40, 2, "post", "tail"), (2, 6, 100 * 90 - 13, 64, 100, 2, "pre", "none")]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("E,H,N,D,B,T,pad,mask", SHAPES)
+def test_tile_kernels_match_the_oracle(E, H, N, D, B, T, pad, mask, dtype):
+    import monarch_attention_b200 as ma
+    from oracle.monarch_oracle import monarch_attention_oracle
+    g = torch.Generator().manual_seed(N * 3 + D)
+    q, k, v = (torch.randn(E, H, N, D, generator=g).to(dtype) for _ in range(3))
+    m = None
+    if mask != "none":
+        m = torch.rand(E, N, generator=g) > (0.3 if mask == "rand" else 0.0)
+        if mask == "block":
+            m[:, B:3 * B] = False
+        if mask == "tail":
+            m[0, N // 3:] = False
+        m[:, 0] = True
+    dev = torch.device("cuda:0")
+    md = None if m is None else m.to(dev)
+    args = [t.to(dev) for t in (q, k, v)]
+    mod = ma.MonarchAttention(B, T, pad, impl="b200-tile")
+    out = mod(*args, md)
+    ref = monarch_attention_oracle(q, k, v, m, T, B, pad == "pre").float()
+    err = ((out.cpu().float() - ref).norm() / ref.norm()).item()
+    assert torch.isfinite(out.float()).all() and err <= (1e-2 if dtype == torch.bfloat16 else 2e-3), err
+    strided = [t.permute(0, 2, 1, 3).contiguous().permute(0, 2, 1, 3) for t in args]
+    assert torch.equal(mod(*strided, md), out)
