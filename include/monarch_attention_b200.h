@@ -133,6 +133,21 @@ MA_B200_API int ma_b200_workspace_layout_of(const ma_b200_problem* p, ma_b200_wo
  * reference: monarch_attention_torch, ma/ma_torch.py:65-108. */
 MA_B200_API int ma_b200_forward(const ma_b200_problem* p, void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same with p->mask pointing to values of another type (MA_B200_MASK_*; p->mask_stride_e counts elements): the
+ * masks the models pass are int64 (text encoders) or float (summarisation), and non-zero means valid whatever the type
+ * (reference: ma/ma_torch.py:96-98). */
+enum {
+  MA_B200_MASK_U8 = 0, /* bytes: bool, int8, uint8 (what ma_b200_forward takes) */
+  MA_B200_MASK_I16 = 1,
+  MA_B200_MASK_I32 = 2,
+  MA_B200_MASK_I64 = 3,
+  MA_B200_MASK_F16 = 4, /* f16 or bf16 */
+  MA_B200_MASK_F32 = 5,
+  MA_B200_MASK_F64 = 6
+};
+MA_B200_API int ma_b200_forward_typed_mask(const ma_b200_problem* p, int mask_type, void* workspace, size_t workspace_bytes,
+                                           void* stream);
+
 /* Same as ma_b200_forward, and additionally records one CUDA event pair per stage launch
  * and, after synchronising the stream, writes the stage durations in milliseconds to
  * stage_ms[0 .. min(n_stage_ms, 2*num_steps) - 1] in launch order (the fused kernel has a single
@@ -156,6 +171,8 @@ typedef struct ma_b200_gradients {
 MA_B200_API size_t ma_b200_backward_workspace_bytes(const ma_b200_problem* p);
 MA_B200_API int ma_b200_backward(const ma_b200_problem* p, const ma_b200_gradients* g, void* workspace,
                                  size_t workspace_bytes, void* stream);
+MA_B200_API int ma_b200_backward_typed_mask(const ma_b200_problem* p, int mask_type, const ma_b200_gradients* g,
+                                            void* workspace, size_t workspace_bytes, void* stream);
 
 /* Synchronise `stream` and read the device-side status flag of the last forward that used
  * this workspace: MA_B200_OK or MA_B200_DEVICE_WAIT_EXPIRED. */

@@ -64,7 +64,7 @@ int validate(const ma_b200_problem* p, bool need_pointers) {
   return MA_B200_OK;
 }
 
-ma::Geometry make_geometry(const ma_b200_problem* p) {
+ma::Geometry make_geometry(const ma_b200_problem* p, int mask_type = MA_B200_MASK_U8) {
   ma::Geometry g;
   memset(&g, 0, sizeof(g));
   g.E = p->E; g.H = p->H; g.N = p->N; g.D = p->D; g.Dv = p->Dv;
@@ -80,6 +80,7 @@ ma::Geometry make_geometry(const ma_b200_problem* p) {
   };
   g.q = view(p->q); g.k = view(p->k); g.v = view(p->v); g.out = view(p->out);
   g.mask = p->mask;
+  g.mask_type = mask_type;
   g.mask_se = p->mask_stride_e;
   return g;
 }
@@ -151,9 +152,18 @@ int layout_of(const ma_b200_problem* p, ma_b200_workspace_layout* L) {
   return MA_B200_OK;
 }
 
-int run_forward(const ma_b200_problem* p, void* workspace, size_t workspace_bytes, void* stream_v, float* stage_ms,
+int check_mask_type(const ma_b200_problem* p, int mask_type) {
+  static const int bytes[] = {1, 2, 4, 8, 2, 4, 8};
+  if (mask_type < MA_B200_MASK_U8 || mask_type > MA_B200_MASK_F64) return fail(MA_B200_INVALID_ARGUMENT, "unknown mask type");
+  if (p != nullptr && reinterpret_cast<uintptr_t>(p->mask) % bytes[mask_type] != 0)
+    return fail(MA_B200_INVALID_ARGUMENT, "mask: pointer not aligned to its element size");
+  return MA_B200_OK;
+}
+
+int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t workspace_bytes, void* stream_v, float* stage_ms,
                 int n_stage_ms) {
   int rc = validate(p, true);
+  if (rc == MA_B200_OK) rc = check_mask_type(p, mask_type);
   if (rc != MA_B200_OK) return rc;
   ma_b200_workspace_layout L;
   rc = layout_of(p, &L);
@@ -165,7 +175,7 @@ int run_forward(const ma_b200_problem* p, void* workspace, size_t workspace_byte
     return fail(MA_B200_WORKSPACE_TOO_SMALL, "workspace has " + std::to_string(workspace_bytes) + " bytes, need " +
                                                  std::to_string(L.total));
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
-  ma::Geometry g = make_geometry(p);
+  ma::Geometry g = make_geometry(p, mask_type);
   char* ws = reinterpret_cast<char*>(workspace);
   g.status = reinterpret_cast<int*>(ws + L.status);
   g.ar = ws + L.ar;
@@ -281,13 +291,17 @@ int ma_b200_workspace_layout_of(const ma_b200_problem* p, ma_b200_workspace_layo
 }
 
 int ma_b200_forward(const ma_b200_problem* p, void* workspace, size_t workspace_bytes, void* stream) {
-  return run_forward(p, workspace, workspace_bytes, stream, nullptr, 0);
+  return run_forward(p, MA_B200_MASK_U8, workspace, workspace_bytes, stream, nullptr, 0);
+}
+
+int ma_b200_forward_typed_mask(const ma_b200_problem* p, int mask_type, void* workspace, size_t workspace_bytes, void* stream) {
+  return run_forward(p, mask_type, workspace, workspace_bytes, stream, nullptr, 0);
 }
 
 int ma_b200_forward_timed(const ma_b200_problem* p, void* workspace, size_t workspace_bytes, void* stream,
                           float* stage_ms, int32_t n_stage_ms) {
   if (stage_ms == nullptr || n_stage_ms <= 0) return fail(MA_B200_INVALID_ARGUMENT, "stage_ms is NULL or empty");
-  return run_forward(p, workspace, workspace_bytes, stream, stage_ms, n_stage_ms);
+  return run_forward(p, MA_B200_MASK_U8, workspace, workspace_bytes, stream, stage_ms, n_stage_ms);
 }
 
 size_t ma_b200_backward_workspace_bytes(const ma_b200_problem* p) {
@@ -303,13 +317,19 @@ size_t ma_b200_backward_workspace_bytes(const ma_b200_problem* p) {
 
 int ma_b200_backward(const ma_b200_problem* p, const ma_b200_gradients* gr, void* workspace, size_t workspace_bytes,
                      void* stream) {
+  return ma_b200_backward_typed_mask(p, MA_B200_MASK_U8, gr, workspace, workspace_bytes, stream);
+}
+
+int ma_b200_backward_typed_mask(const ma_b200_problem* p, int mask_type, const ma_b200_gradients* gr, void* workspace,
+                                size_t workspace_bytes, void* stream) {
   if (p == nullptr || gr == nullptr) return fail(MA_B200_INVALID_ARGUMENT, "problem or gradients is NULL");
   ma_b200_problem q = *p;
   q.out = gr->grad_out;  // takes the output's place in the checks of pointers and alignment
   if (q.out.stride_n < q.Dv) q.out.stride_n = q.Dv;  // (read only: rows may repeat)
   int rc = validate(&q, true);
+  if (rc == MA_B200_OK) rc = check_mask_type(&q, mask_type);
   if (rc != MA_B200_OK) return rc;
-  ma::Geometry g = make_geometry(&q);
+  ma::Geometry g = make_geometry(&q, mask_type);
   g.out.sn = gr->grad_out.stride_n;
   const char* why = "";
   if (!ma::backward_supported(g, p->qk_dtype, p->v_dtype, &why))

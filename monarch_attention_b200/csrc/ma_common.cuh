@@ -31,8 +31,9 @@ struct Geometry {
   int T;
   float sm_scale;  // (float)(1/sqrt(D))
   View4 q, k, v, out;
-  const uint8_t* mask;  // (E,N) bytes, non-zero = valid; or nullptr
-  long long mask_se;
+  const uint8_t* mask;  // (E,N) values of mask_type, non-zero = valid; or nullptr
+  long long mask_se;    // elements
+  int mask_type;        // MA_B200_MASK_*
   // stage-to-stage state (workspace)
   void* ar;   // (EH, M, B, D)  qk dtype
   float* cr;  // (EH, M, B)
@@ -84,6 +85,22 @@ inline cudaError_t allow_dynamic_smem(const void* fn, size_t bytes) {
   e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e == cudaSuccess) have = bytes;
   return e;
+}
+
+// Whether the mask lets token n of batch element e through.  The callers' masks come as booleans, integers or floats
+// (-0.0 is zero); reading them as they are saves a conversion kernel in front of every call.
+__device__ __forceinline__ bool mask_lets(const Geometry& g, int e, int n) {
+  if (g.mask == nullptr) return true;
+  const long long i = (long long)e * g.mask_se + n;
+  switch (g.mask_type) {
+    case MA_B200_MASK_I64: return reinterpret_cast<const unsigned long long*>(g.mask)[i] != 0;
+    case MA_B200_MASK_F32: return (reinterpret_cast<const uint32_t*>(g.mask)[i] & 0x7fffffffu) != 0;
+    case MA_B200_MASK_I32: return reinterpret_cast<const uint32_t*>(g.mask)[i] != 0;
+    case MA_B200_MASK_F16: return (reinterpret_cast<const uint16_t*>(g.mask)[i] & 0x7fffu) != 0;
+    case MA_B200_MASK_I16: return reinterpret_cast<const uint16_t*>(g.mask)[i] != 0;
+    case MA_B200_MASK_F64: return (reinterpret_cast<const unsigned long long*>(g.mask)[i] << 1) != 0;
+    default: return g.mask[i] != 0;
+  }
 }
 
 // Host-side launchers implemented by the kernel translation units.

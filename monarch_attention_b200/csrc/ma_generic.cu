@@ -90,7 +90,7 @@ __device__ __forceinline__ void stage_dense_rows(float* dst, const T* src, int r
 __device__ __forceinline__ bool token_valid(const Geometry& g, int e, int p) {
   int n = p - g.pad_off;
   if (n < 0 || n >= g.N) return false;
-  return g.mask == nullptr || g.mask[(long long)e * g.mask_se + n] != 0;
+  return mask_lets(g, e, n);
 }
 
 // ---------------------------------------------------------------------------------

@@ -96,7 +96,7 @@ __device__ __forceinline__ float rcp_fast(float x) {
 __device__ __forceinline__ bool token_valid(const Geometry& g, int e, int p) {
   const int n = p - g.pad_off;
   if (n < 0 || n >= g.N) return false;
-  return g.mask == nullptr || g.mask[(long long)e * g.mask_se + n] != 0;
+  return mask_lets(g, e, n);
 }
 
 // NK: key columns of a row's unit, rounded up: 64 (two units per tile), 128 or 256.
@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(NK))
           v[k] = x < units && r < keys ? g.cr[((long long)w.eh * M + x) * B + r] : 1.0f;
         } else {
           const int n = r * B + column_start(x);
-          v[k] = x < units && r < keys && n < g.N && (g.mask == nullptr || g.mask[(long long)w.e * g.mask_se + n] != 0) ? 1.0f : 0.0f;
+          v[k] = x < units && r < keys && n < g.N && mask_lets(g, w.e, n) ? 1.0f : 0.0f;
         }
       }
     };

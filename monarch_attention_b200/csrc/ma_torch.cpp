@@ -59,11 +59,24 @@ void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const optio
                       "attention_mask must have shape (batch, tokens) = (", q.size(0), ", ", q.size(2), ")");
 }
 
-// One byte per token, non-zero = valid, unit inner stride (any mask type: non-zero counts as valid).
-Tensor mask_bytes(const Tensor& mask, const Tensor& q) {
+int mask_type(at::ScalarType t) {
+  switch (t) {
+    case at::kBool: case at::kByte: case at::kChar: return MA_B200_MASK_U8;
+    case at::kShort: return MA_B200_MASK_I16;
+    case at::kInt: return MA_B200_MASK_I32;
+    case at::kLong: return MA_B200_MASK_I64;
+    case at::kHalf: case at::kBFloat16: return MA_B200_MASK_F16;
+    case at::kFloat: return MA_B200_MASK_F32;
+    case at::kDouble: return MA_B200_MASK_F64;
+    default: return -1;
+  }
+}
+
+// A mask the kernels can read (non-zero counts as valid): on the queries' device, unit inner stride.
+Tensor readable_mask(const Tensor& mask, const Tensor& q) {
   Tensor m = mask.device() == q.device() ? mask : mask.to(q.device());
-  if (m.scalar_type() != at::kBool) m = m.ne(0);
-  return m.stride(-1) == 1 ? m : m.contiguous();
+  if (mask_type(m.scalar_type()) < 0) m = m.ne(0);
+  return m.stride(-1) == 1 || m.size(-1) == 1 ? m : m.contiguous();
 }
 
 struct Call {
@@ -108,7 +121,7 @@ Tensor run_kernels(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, c
   raise_for_status(ma_b200_workspace_layout_of(&p, &layout));
   const auto stream = c10::cuda::getCurrentCUDAStream();
   const c10::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate(layout.total);
-  raise_for_status(ma_b200_forward(&p, ws.get(), layout.total, stream.stream()));
+  raise_for_status(ma_b200_forward_typed_mask(&p, mask.defined() ? mask_type(mask.scalar_type()) : MA_B200_MASK_U8, ws.get(), layout.total, stream.stream()));
   return out;
 }
 
@@ -155,7 +168,7 @@ struct AttentionFunction : torch::autograd::Function<AttentionFunction> {
     if (ctx->needs_input_grad(2)) { dv = at::empty_like(v); g.dv = view4(dv); }
     const auto stream = c10::cuda::getCurrentCUDAStream();
     const c10::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate(need);
-    raise_for_status(ma_b200_backward(&p, &g, ws.get(), need, stream.stream()));
+    raise_for_status(ma_b200_backward_typed_mask(&p, mask.defined() ? mask_type(mask.scalar_type()) : MA_B200_MASK_U8, &g, ws.get(), need, stream.stream()));
     return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
@@ -191,9 +204,9 @@ PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const bool grad = at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad());
     TORCH_CHECK_VALUE(!grad || !out.defined(), "out= cannot be combined with inputs that require a gradient");
     if (!grad) {
-      result = run_kernels(q, k, v, mask_in.has_value() ? mask_bytes(*mask_in, q) : Tensor(), c, out, token_major);
+      result = run_kernels(q, k, v, mask_in.has_value() ? readable_mask(*mask_in, q) : Tensor(), c, out, token_major);
     } else if (backward_kernels_take(q, k, v, c)) {
-      result = AttentionFunction::apply(q, k, v, mask_in.has_value() ? optional<Tensor>(mask_bytes(*mask_in, q)) : std::nullopt, c.T, c.B, c.pre_pad,
+      result = AttentionFunction::apply(q, k, v, mask_in.has_value() ? optional<Tensor>(readable_mask(*mask_in, q)) : std::nullopt, c.T, c.B, c.pre_pad,
                                         (int64_t)c.kernel, token_major);
     }
   }

@@ -138,7 +138,7 @@ __device__ __forceinline__ void clear_status(const Geometry& g) {
 __device__ __forceinline__ bool pos_valid(const Geometry& g, int e, int p) {
   const int n = p - g.pad_off;
   if (n < 0 || n >= g.N) return false;
-  return g.mask == nullptr || g.mask[(long long)e * g.mask_se + n] != 0;
+  return mask_lets(g, e, n);
 }
 // Row of a user tensor for padded position p, given the (e, h) base pointer: nullptr for padding.
 template <typename T>
