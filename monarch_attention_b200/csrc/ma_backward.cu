@@ -36,7 +36,7 @@ struct BackwardArgs {
   View4 dz, dq, dk, dv;  // user tensors; dq / dk / dv may have a null pointer (not wanted)
   void *dal, *dy, *dar;  // (EH, B, M, D), (EH, B, M, D), (EH, M, B, D), storage type
   float *dcl, *dcr;      // (EH, B, M), (EH, M, B)
-  float *dq_acc, *dk_acc;  // (EH, M*B, D) in padded token order
+  float *dq_acc, *dk_acc;  // (EH, B, M, D) and (EH, M, B, D): the tiles that add to them own consecutive rows
   int first;             // right-factor: first iteration (ar = q, cr = 1)
   int accumulate;        // right-factor: dk_acc holds the later iterations' sum
 };
@@ -69,6 +69,15 @@ __device__ __forceinline__ void warp_gemm_pv_add(float (&o)[DP / 8][4], const Fa
       Tile<T>::mma(o[2 * np], o[2 * np + 1], a, b);
     }
   }
+}
+
+// Asks for the 16 fp32 rows a warp will add to much later (each lane for half a row or less), so that the addition does
+// not wait for memory: the kernels are bound by such waits, not by bandwidth or arithmetic.
+template <typename RowFn>
+__device__ __forceinline__ void prefetch_rows_f32(RowFn row_ptr, int D, int lane) {
+  const float* p = row_ptr(lane >> 1);
+  if (p == nullptr) return;
+  for (int c = (lane & 1) * 32; c < D; c += 64) asm volatile("prefetch.global.L1 [%0];" ::"l"(p + c));
 }
 
 template <int DP>
@@ -160,6 +169,18 @@ __global__ void __launch_bounds__(2 * KP) backward_column_kernel(const BackwardA
     load_rows<T, RowPieces<T, DP>::n>(sX, PITCH, M, KP, D, reinterpret_cast<const T*>(a.dar) + (long long)eh * M * B * D, j, B, M * B, D,
                                       tid, nth, g.q.ptr);
   }
+  const int warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t = lane & 3, row0 = warp * 16;
+  const int l_lo = row0 + gq, l_hi = l_lo + 8;
+  float ok_lo = 1.f, ok_hi = 1.f;
+  auto dq_row = [&](int r) -> float* {
+    const int l = row0 + r;
+    return l < M ? a.dq_acc + (((long long)eh * B + j) * M + l) * D : nullptr;
+  };
+  if (!OUT) {
+    ok_lo = pos_valid(g, e, l_lo * B + j) ? 1.f : 0.f;
+    ok_hi = pos_valid(g, e, l_hi * B + j) ? 1.f : 0.f;
+    prefetch_rows_f32(dq_row, D, lane);
+  }
   for (int i = tid; i < KP; i += nth) {
     nbias[i] = i < M ? -g.cl[col + i] : -INFINITY;
     if (!OUT) dcrs[i] = i < M ? a.dcr[((long long)eh * M + i) * B + j] : 0.f;
@@ -167,17 +188,10 @@ __global__ void __launch_bounds__(2 * KP) backward_column_kernel(const BackwardA
   tiles_commit_and_wait();
   __syncthreads();
 
-  const int warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t = lane & 3, row0 = warp * 16;
   {
     float s[KP / 8][4], d[KP / 8][4];
     column_softmax<T, KP, DP, PITCH>(s, sQ + row0 * PITCH, sAL, nbias, lane);
     warp_gemm_abt<T, KP, DP, PITCH>(d, (OUT ? sDZ : sQ) + row0 * PITCH, sX, lane);
-    const int l_lo = row0 + gq, l_hi = l_lo + 8;
-    float ok_lo = 1.f, ok_hi = 1.f;
-    if (!OUT) {
-      ok_lo = pos_valid(g, e, l_lo * B + j) ? 1.f : 0.f;
-      ok_hi = pos_valid(g, e, l_hi * B + j) ? 1.f : 0.f;
-    }
     float de_lo = 0.f, de_hi = 0.f;
 #pragma unroll
     for (int nt = 0; nt < KP / 8; ++nt) {
@@ -224,10 +238,7 @@ __global__ void __launch_bounds__(2 * KP) backward_column_kernel(const BackwardA
     Factor<T, KP> f;
     f.set(d);
     warp_gemm_pv_add<T, KP, DP, PITCH>(o, f, sAL, lane);
-    update_rows_f32<DP>(o, [&](int r) -> float* {
-      const int l = row0 + r;
-      return l < M ? a.dq_acc + (((long long)eh * M + l) * B + j) * D : nullptr;
-    }, D, lane, !OUT);
+    update_rows_f32<DP>(o, dq_row, D, lane, !OUT);
   }
   __syncthreads();
 
@@ -260,11 +271,11 @@ __global__ void __launch_bounds__(2 * KP) backward_column_kernel(const BackwardA
 // ---------------------------------------------------------------------------------------------------
 template <typename T, int KP, int DP>
 constexpr size_t right_elems(bool with_v, int RP) {
-  return (size_t)(3 * RP + KP + (with_v ? KP + RP : 0)) * (DP + 8) + (size_t)2 * RP * (KP + 8) + (size_t)kF<T> * KP;
+  return (size_t)(2 * RP + KP + (with_v ? KP + RP : 0)) * (DP + 8) + (size_t)2 * RP * (KP + 8) + (size_t)kF<T> * KP;
 }
 
 template <typename T, int KP, int DP, bool WITH_V>
-__global__ void __launch_bounds__(2 * KP) backward_right_kernel(const BackwardArgs a) {
+__global__ void __launch_bounds__(2 * KP, KP == 32 && sizeof(T) == 2 ? 10 : 1) backward_right_kernel(const BackwardArgs a) {
   constexpr int PITCH = DP + 8, PP = KP + 8;
   extern __shared__ __align__(16) uint8_t smem[];
   const Geometry& g = a.g;
@@ -272,8 +283,7 @@ __global__ void __launch_bounds__(2 * KP) backward_right_kernel(const BackwardAr
   const int B = g.B, M = g.M, D = g.D, tid = threadIdx.x, nth = blockDim.x, RP = nth >> 1;
   T* sA = reinterpret_cast<T*>(smem);
   T* sDAL = sA + RP * PITCH;
-  T* sOut = sDAL + RP * PITCH;                    // staging of the stores
-  T* sK = sOut + RP * PITCH;
+  T* sK = sDAL + RP * PITCH;
   T* sV = sK + KP * PITCH;                        // WITH_V only, as sDY
   T* sDY = sV + (WITH_V ? KP * PITCH : 0);
   T* sP = sDY + (WITH_V ? RP * PITCH : 0);        // [RP][PP] factor
@@ -294,13 +304,22 @@ __global__ void __launch_bounds__(2 * KP) backward_right_kernel(const BackwardAr
     load_rows<T, RowPieces<T, DP>::n>(sDY, PITCH, B, RP, D, reinterpret_cast<const T*>(a.dy) + (st + m) * D, 0, 1, B, (long long)M * D,
                                       tid, nth, g.q.ptr);
   }
+  const int warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t = lane & 3, row0 = warp * 16;
+  const int r_lo = row0 + gq, r_hi = r_lo + 8;
+  const float cr_lo = (a.first || r_lo >= B ? 1.0f : g.cr[blk + r_lo]) + kEps;
+  const float cr_hi = (a.first || r_hi >= B ? 1.0f : g.cr[blk + r_hi]) + kEps;
+  const float dcl_lo = r_lo < B ? a.dcl[st + (long long)r_lo * M + m] : 0.f;
+  const float dcl_hi = r_hi < B ? a.dcl[st + (long long)r_hi * M + m] : 0.f;
+  auto dq_row = [&](int r) -> float* { return row0 + r < B ? a.dq_acc + (st + (long long)(row0 + r) * M + m) * D : nullptr; };
+  auto dk_row = [&](int r) -> float* { return row0 + r < B ? a.dk_acc + (blk + row0 + r) * D : nullptr; };
+  if (a.first) prefetch_rows_f32(dq_row, D, lane);
+  if (a.accumulate) prefetch_rows_f32(dk_row, D, lane);
   for (int i = tid; i < KP; i += nth) kbias[i] = (i < B && pos_valid(g, e, m * B + i)) ? 0.f : -INFINITY;
   tiles_commit_and_wait();
   __syncthreads();
 
-  const int warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t = lane & 3, row0 = warp * 16;
+  float row_grad[DP / 8][4];  // dar, or dq of the first stage: stored after the next barrier, from where the key tile was
   {
-    const int r_lo = row0 + gq, r_hi = r_lo + 8;
     float s[KP / 8][4], d[KP / 8][4];
     warp_gemm_abt<T, KP, DP, PITCH>(d, sDAL + row0 * PITCH, sK, lane);
 #pragma unroll
@@ -315,10 +334,6 @@ __global__ void __launch_bounds__(2 * KP) backward_right_kernel(const BackwardAr
       }
     }
     warp_gemm_abt<T, KP, DP, PITCH>(s, sA + row0 * PITCH, sK, lane);
-    const float cr_lo = (a.first || r_lo >= B ? 1.0f : g.cr[blk + r_lo]) + kEps;
-    const float cr_hi = (a.first || r_hi >= B ? 1.0f : g.cr[blk + r_hi]) + kEps;
-    const float dcl_lo = r_lo < B ? a.dcl[st + (long long)r_lo * M + m] : 0.f;
-    const float dcl_hi = r_hi < B ? a.dcl[st + (long long)r_hi * M + m] : 0.f;
     const float c_lo = g.sm_scale / cr_lo, c_hi = g.sm_scale / cr_hi;
     float mx_lo = -INFINITY, mx_hi = -INFINITY;
 #pragma unroll
@@ -373,29 +388,26 @@ __global__ void __launch_bounds__(2 * KP) backward_right_kernel(const BackwardAr
       Tile<T>::store_pair(sG + r_lo * PP + c, d[nt][0], d[nt][1]);
       Tile<T>::store_pair(sG + r_hi * PP + c, d[nt][2], d[nt][3]);
     }
-    float o[DP / 8][4];
-    zero_acc<DP>(o);
-    {
-      Factor<T, KP> f;
-      f.set(d);
-      warp_gemm_pv_add<T, KP, DP, PITCH>(o, f, sK, lane);
-    }
-    T* stage = sOut + row0 * PITCH;
-    if (a.first) {
-      add_rows_f32<DP>(o, [&](int r) -> const float* { return row0 + r < B ? a.dq_acc + (blk + row0 + r) * D : nullptr; }, D, lane);
-      store_rows<T, DP, PITCH>(o, stage, [&](int r) -> T* {
-        return row0 + r < B ? user_row_or_null<T>(a.dq, g, e, h, m * B + row0 + r) : nullptr;
-      }, D, lane, 1.0f, false);
-    } else {
-      T* dar = reinterpret_cast<T*>(a.dar) + blk * D;
-      store_rows<T, DP, PITCH>(o, stage, [&](int r) -> T* { return row0 + r < B ? dar + (long long)(row0 + r) * D : nullptr; }, D, lane,
-                               1.0f, false);
-    }
+    zero_acc<DP>(row_grad);
+    Factor<T, KP> f;
+    f.set(d);
+    warp_gemm_pv_add<T, KP, DP, PITCH>(row_grad, f, sK, lane);
   }
   __syncthreads();
 
+  T* stage = sK + row0 * PITCH;  // (the key tile has been read)
+  if (a.first) {
+    add_rows_f32<DP>(row_grad, dq_row, D, lane);
+    store_rows<T, DP, PITCH>(row_grad, stage, [&](int r) -> T* {
+      return row0 + r < B ? user_row_or_null<T>(a.dq, g, e, h, m * B + row0 + r) : nullptr;
+    }, D, lane, 1.0f, false);
+  } else {
+    T* dar = reinterpret_cast<T*>(a.dar) + blk * D;
+    store_rows<T, DP, PITCH>(row_grad, stage, [&](int r) -> T* { return row0 + r < B ? dar + (long long)(row0 + r) * D : nullptr; }, D,
+                             lane, 1.0f, false);
+  }
+
   // keys i of this warp
-  T* stage = sOut + row0 * PITCH;
   {
     float o[DP / 8][4];
     zero_acc<DP>(o);
@@ -405,14 +417,13 @@ __global__ void __launch_bounds__(2 * KP) backward_right_kernel(const BackwardAr
       o[nt][0] *= g.sm_scale; o[nt][1] *= g.sm_scale; o[nt][2] *= g.sm_scale; o[nt][3] *= g.sm_scale;
     }
     warp_gemm_atb<T, DP, PITCH>(o, sG + row0, PP, sA, RP / 16, lane);
-    auto acc_row = [&](int r) -> float* { return row0 + r < B ? a.dk_acc + (blk + row0 + r) * D : nullptr; };
     if (a.first) {
-      if (a.accumulate) add_rows_f32<DP>(o, acc_row, D, lane);
+      if (a.accumulate) add_rows_f32<DP>(o, dk_row, D, lane);
       store_rows<T, DP, PITCH>(o, stage, [&](int r) -> T* {
         return row0 + r < B ? user_row_or_null<T>(a.dk, g, e, h, m * B + row0 + r) : nullptr;
       }, D, lane, 1.0f, false);
     } else {
-      update_rows_f32<DP>(o, acc_row, D, lane, a.accumulate != 0);
+      update_rows_f32<DP>(o, dk_row, D, lane, a.accumulate != 0);
     }
   }
   if (WITH_V) {
