@@ -190,8 +190,10 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
   // Status word and stage-completion counters start at zero.  The stage kernels that wait for nothing clear the
   // status word themselves: a memset in front of them is 1.5 us on the stream, as much as a small kernel.
   cudaError_t ce = cudaSuccess;
-  if (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3 && L.kernel != MA_B200_KERNEL_HEAD_RESIDENT &&
-      L.kernel != MA_B200_KERNEL_TILE) {
+  // (with per-stage times wanted, the tile kernels run one launch per stage)
+  const bool flow = L.kernel == MA_B200_KERNEL_TILE && stage_ms == nullptr && ma::flow_supported(g);
+  if (flow || (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3 && L.kernel != MA_B200_KERNEL_HEAD_RESIDENT &&
+               L.kernel != MA_B200_KERNEL_TILE)) {
     ce = cudaMemsetAsync(ws + L.status, 0, L.ar - L.status, stream);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(status, counters)");
   }
@@ -243,6 +245,9 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
     if (ce != cudaSuccess) rc = cuda_fail(ce, "one-CTA-per-head kernel");
     if (ev != nullptr)
       for (int i = 1; i <= n_stages; ++i) cudaEventRecord(ev[i], stream);
+  } else if (flow) {
+    ce = ma::launch_flow(g, p->qk_dtype, counters, host_status, stream);
+    if (ce != cudaSuccess) rc = cuda_fail(ce, "tile kernels in one launch");
   } else if (L.kernel == MA_B200_KERNEL_TCGEN05) {
     // every stage in one persistent launch
     ce = ma::launch_fused(plan, g, counters, 0, n_stages, 1, stream);

@@ -151,6 +151,10 @@ int* host_status_word(int device);
 // tcgen05 stage kernels, one 128-row tile per CTA: block size and count up to 256, D <= 64, masks and padding (ma_tile.cu).
 bool tile_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
 cudaError_t launch_tile_stage(const Geometry& g, int dtype, StageKind kind, bool first, int* host_status, cudaStream_t stream);
+// Their single-launch form, all stages of a call, for block size and count up to 128 (ma_flow.cu); counters: (E*H, 2T)
+// zeroed ints.
+bool flow_supported(const Geometry& g);
+cudaError_t launch_flow(const Geometry& g, int dtype, int* counters, int* host_status, cudaStream_t stream);
 // Code of a bounded device-side wait that gave up on `device` since the last poll (0 = none); reads a mapped
 // host word, so it needs no synchronisation.
 int fused_poll_status(int device);
