@@ -52,7 +52,7 @@ enum {
 /* Element types.  q and k share qk_dtype; v and out share v_dtype. */
 enum { MA_B200_F32 = 0, MA_B200_BF16 = 1, MA_B200_F16 = 2 };
 
-/* Kernel families.  AUTO picks the fused tcgen05 kernel when the problem fits it, else the
+/* Kernel families.  AUTO picks the fused tcgen05 kernel when the problem fits it and is small, else the
  * head-resident kernel, else the tcgen05 tile kernels, else the warp-level tensor-core kernels (16-bit or fp32), else the generic kernels.
  *   GENERIC        SIMT stage kernels, any shape / dtype / mask (2T launches)
  *   TCGEN05        persistent tcgen05 kernel, all 2T stages in one launch: 16-bit inputs,
@@ -69,7 +69,7 @@ enum { MA_B200_F32 = 0, MA_B200_BF16 = 1, MA_B200_F16 = 2 };
  *   HEAD_RESIDENT  16-bit inputs, block size and block count up to 32, D <= 80 (multiple of 8): one CTA
  *                  or cluster per head, all stages in one launch, the head's state on chip where it fits
  *   TILE           tcgen05 stage kernels, one 128-row tile per CTA: 16-bit inputs, block size and block count
- *                  up to 256, D <= 64 (multiple of 8), masks and padding (2T launches) */
+ *                  up to 256, D <= 64 (multiple of 8), masks and padding (one launch up to 128, else 2T) */
 enum {
   MA_B200_KERNEL_AUTO = 0,
   MA_B200_KERNEL_GENERIC = 1,

@@ -114,10 +114,18 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, int* kernel)
   // Heads narrower than 24 leave most of a 16-wide contraction step of the fp32 tensor path padded or give it one
   // step per tile; the thread-per-logit kernels are as fast there.
   const bool tf32_pays = tf32_ok && g.D >= 24;
+  // The pipelined fused kernel takes a tile through a stage in 5 us, the tile kernels in 7 to 8, but those do 1.2 to 1.3
+  // times as many tiles in a time: the fused kernel where a stage has no more tiles than fit the GPU at once (592; measured
+  // at 512 tiles 41 against 43 us, at 1024 tiles 74 against 68), half as many when there is one iteration only.
+  const bool few_tiles = (long long)p->E * p->H * p->N / 128 * (p->num_steps == 1 ? 2 : 1) <= 592;
   if (p->kernel == MA_B200_KERNEL_AUTO)
-    // (the one-CTA-per-head kernel is selectable but not preferred: on the ViT / RoBERTa shapes it
-    // measured slower than the two staged launches - these tiny tiles are instruction-bound)
-    *kernel = tc_ok ? MA_B200_KERNEL_TCGEN05 : resident_ok ? MA_B200_KERNEL_HEAD_RESIDENT : tile_ok ? MA_B200_KERNEL_TILE : (warp_ok ? MA_B200_KERNEL_WARP_MMA : (tf32_pays ? MA_B200_KERNEL_TF32X3 : MA_B200_KERNEL_GENERIC));
+    // (the older one-CTA-per-head kernel, HEAD_FUSED, is selectable but never preferred)
+    *kernel = tc_ok && few_tiles ? MA_B200_KERNEL_TCGEN05
+              : resident_ok      ? MA_B200_KERNEL_HEAD_RESIDENT
+              : tile_ok          ? MA_B200_KERNEL_TILE
+              : warp_ok          ? MA_B200_KERNEL_WARP_MMA
+              : tf32_pays        ? MA_B200_KERNEL_TF32X3
+                                 : MA_B200_KERNEL_GENERIC;
   else *kernel = p->kernel;
   if (*kernel == MA_B200_KERNEL_GENERIC) {
     const size_t need = ma::generic_stage_smem_bytes(g, g.B > g.M ? ma::kStageRight : ma::kStageLeft);
