@@ -85,6 +85,24 @@ ma::Geometry make_geometry(const ma_b200_problem* p, int mask_type = MA_B200_MAS
   return g;
 }
 
+// Whether the warp-level kernels are expected to take a problem faster than the tcgen05 tile kernels: those work on tiles of
+// 128 x 64 or 128 x 128 whatever the blocks fill of them, so that blocks just above 32, a long side beside a short one,
+// narrow heads and few heads are better off with 16-row warps and two launches.  Microseconds of one iteration, from a
+// sweep of blocks and counts of 16 to 200, 4 to 256 heads and widths 32 and 64: a tile takes 12.5 ns of the GPU's time and an
+// iteration 18.6 us at the least (8 beside the tiles' own time); a padded element of a warp-level tile takes 2.4 ps (1.7 in
+// heads of up to 32), two launches 6 us.
+bool warp_beats_tiles(const ma::Geometry& g) {
+  if (g.B > 128 || g.M > 128) return false;  // (the warp-level kernels then walk a row twice: never the faster ones)
+  const double heads = (double)g.E * g.H;
+  auto up16 = [](int x) { return (x + 15) & ~15; };
+  auto keys = [](int x) { return x <= 16 ? 16 : x <= 32 ? 32 : x <= 64 ? 64 : 128; };
+  const double elements = heads * ((double)g.M * up16(g.B) * keys(g.B) + (double)g.B * up16(g.M) * keys(g.M));
+  const double tiles = heads * ((g.B <= 64 ? (g.M + 1) / 2 : g.M) + (g.M <= 64 ? (g.B + 1) / 2 : g.B));
+  const double warp_us = 6.0 + elements * (g.D <= 32 ? 1.7e-6 : 2.4e-6);
+  const double tile_us = tiles * 12.5e-3 + 8.0;
+  return warp_us < (tile_us > 18.6 ? tile_us : 18.6);
+}
+
 int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, int* kernel) {
   const char* why = "";
   const bool tc_ok = ma::tc_supported(g, p->qk_dtype, p->v_dtype, &why);
@@ -118,11 +136,15 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, int* kernel)
   // times as many tiles in a time: the fused kernel where a stage has no more tiles than fit the GPU at once (592; measured
   // at 512 tiles 41 against 43 us, at 1024 tiles 74 against 68), half as many when there is one iteration only.
   const bool few_tiles = (long long)p->E * p->H * p->N / 128 * (p->num_steps == 1 ? 2 : 1) <= 592;
+  // Head widths other than 64 and 72 have one tile size for both kinds of stage in the head-resident kernel: with one side of
+  // up to 16 beside a longer one, and heads enough to fill the GPU, the warp-level kernels pad less (300 heads of 10 x 30 x 80:
+  // 68 against 88 us).
+  const bool lopsided = (g.B <= 16) != (g.M <= 16) && g.D != 64 && g.D != 72 && (long long)p->E * p->H > 148;
   if (p->kernel == MA_B200_KERNEL_AUTO)
     // (the older one-CTA-per-head kernel, HEAD_FUSED, is selectable but never preferred)
     *kernel = tc_ok && few_tiles ? MA_B200_KERNEL_TCGEN05
-              : resident_ok      ? MA_B200_KERNEL_HEAD_RESIDENT
-              : tile_ok          ? MA_B200_KERNEL_TILE
+              : resident_ok && !lopsided ? MA_B200_KERNEL_HEAD_RESIDENT
+              : tile_ok && !(warp_ok && warp_beats_tiles(g)) ? MA_B200_KERNEL_TILE
               : warp_ok          ? MA_B200_KERNEL_WARP_MMA
               : tf32_pays        ? MA_B200_KERNEL_TF32X3
                                  : MA_B200_KERNEL_GENERIC;
