@@ -144,6 +144,7 @@ constexpr size_t column_elems(bool out, int RP) {
 template <typename T, int KP, int DP, bool OUT>
 __global__ void __launch_bounds__(2 * KP) backward_column_kernel(const BackwardArgs a) {
   constexpr int PITCH = DP + 8, PP = KP + 8;
+  stage_begin();
   extern __shared__ __align__(16) uint8_t smem[];
   const Geometry& g = a.g;
   const int eh = blockIdx.y, e = eh / g.H, h = eh - e * g.H, j = blockIdx.x;
@@ -277,6 +278,7 @@ constexpr size_t right_elems(bool with_v, int RP) {
 template <typename T, int KP, int DP, bool WITH_V>
 __global__ void __launch_bounds__(2 * KP, KP == 32 && sizeof(T) == 2 ? 10 : 1) backward_right_kernel(const BackwardArgs a) {
   constexpr int PITCH = DP + 8, PP = KP + 8;
+  stage_begin();
   extern __shared__ __align__(16) uint8_t smem[];
   const Geometry& g = a.g;
   const int eh = blockIdx.y, e = eh / g.H, h = eh - e * g.H, m = blockIdx.x;
@@ -464,7 +466,7 @@ cudaError_t backward_launch(const BackwardArgs& a, BackwardStage st, size_t* sme
   if (const cudaError_t e = allow_dynamic_smem(fn, smem); e != cudaSuccess) return e;
   const int rows = right ? g.B : g.M;
   void* args[] = {(void*)&a};
-  return cudaLaunchKernel(fn, dim3(right ? g.M : g.B, g.E * g.H), dim3(2 * ((rows + 15) & ~15)), args, smem, stream);
+  return launch_stage(fn, dim3(right ? g.M : g.B, g.E * g.H), dim3(2 * ((rows + 15) & ~15)), args, smem, true, stream);
 }
 
 template <typename T, int KP>

@@ -103,6 +103,29 @@ __device__ __forceinline__ bool mask_lets(const Geometry& g, int e, int n) {
   }
 }
 
+// A stage kernel of a call after the first one: its CTAs are brought up under the tail of the stage before, and each waits at
+// its start (stage_begin) until that stage is complete and its stores are visible.  (256 fp32 tokens, two launches: 15.4 to
+// 13.3 us; six launches 84 to 75.  The tcgen05 tile kernels lost by it: their early CTAs took instruction fetch from the
+// running stage.)
+inline cudaError_t launch_stage(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, bool overlap, cudaStream_t stream) {
+  if (!overlap) return cudaLaunchKernel(fn, grid, block, args, smem, stream);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+__device__ __forceinline__ void stage_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Host-side launchers implemented by the kernel translation units.
 // Each returns cudaSuccess or the launch error.
 // Test hook: 1 = the generic family always runs its general (warp-per-row) form.
