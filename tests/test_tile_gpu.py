@@ -43,3 +43,20 @@ def test_tile_kernels_match_the_oracle(E, H, N, D, B, T, pad, mask, dtype):
     assert torch.isfinite(out.float()).all() and err <= (1e-2 if dtype == torch.bfloat16 else 2e-3), err
     strided = [t.permute(0, 2, 1, 3).contiguous().permute(0, 2, 1, 3) for t in args]
     assert torch.equal(mod(*strided, md), out)
+
+
+@pytest.mark.parametrize("H,B,M,T", [(1, 64, 64, 6), (2, 64, 60, 5), (1, 128, 128, 4), (3, 40, 100, 5)])
+def test_single_launch_stages_read_what_the_stage_before_wrote(H, B, M, T):
+    """Few heads and many iterations: in the single launch every tile waits for the stage before, and its row vectors (cl, cr)
+    are read by all lanes of a warp of which one did the waiting.  Two alternating inputs leave different vectors in the same
+    workspace, so a value read too early shows as a difference between calls."""
+    import monarch_attention_b200 as ma
+    g = torch.Generator().manual_seed(B + T)
+    dev = torch.device("cuda:0")
+    mod = ma.MonarchAttention(B, T, "post", impl="b200-tile")
+    inputs = [[torch.randn(1, H, B * M, 64, generator=g).to(torch.bfloat16).to(dev) for _ in range(3)] for _ in range(2)]
+    want = [mod(*x) for x in inputs]
+    assert all(torch.isfinite(w.float()).all() for w in want)
+    for _ in range(10):
+        for x, w in zip(inputs, want):
+            assert torch.equal(mod(*x), w)
