@@ -129,6 +129,13 @@ MA_B200_API size_t ma_b200_workspace_bytes(const ma_b200_problem* p);
 /* Fill *layout; returns MA_B200_OK or an error code. */
 MA_B200_API int ma_b200_workspace_layout_of(const ma_b200_problem* p, ma_b200_workspace_layout* layout);
 
+/* The family (MA_B200_KERNEL_*) that p->kernel = AUTO takes for a call with `heads` (batch, head) pairs of which `part` is
+ * some; 0 on an invalid problem.  AUTO goes by the shape of a head and by the number of heads in the call, and families
+ * differ in the last bits of a result.  Whoever cuts a call into parts (chunks of heads, shards on several GPUs) and wants
+ * the bits of the undivided call asks here once and sets part->kernel to the answer.  `part`: sizes, strides and pointers of
+ * one part (with NULL pointers alignment is taken for granted); only whether mask is NULL is looked at. */
+MA_B200_API int ma_b200_kernel_of_part(const ma_b200_problem* part, int64_t heads);
+
 /* Enqueue the forward pass on `stream` (a cudaStream_t / CUstream; NULL = default stream).
  * reference: monarch_attention_torch, ma/ma_torch.py:65-108. */
 MA_B200_API int ma_b200_forward(const ma_b200_problem* p, void* workspace, size_t workspace_bytes, void* stream);

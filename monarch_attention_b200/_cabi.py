@@ -22,7 +22,7 @@ OK, INVALID_ARGUMENT, UNSUPPORTED, CUDA_ERROR, DEVICE_WAIT_EXPIRED, WORKSPACE_TO
 LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libmonarch_attention_b200.so")
 
 EXPORTS = (
-    "ma_b200_workspace_bytes", "ma_b200_workspace_layout_of", "ma_b200_forward", "ma_b200_forward_timed",
+    "ma_b200_workspace_bytes", "ma_b200_workspace_layout_of", "ma_b200_kernel_of_part", "ma_b200_forward", "ma_b200_forward_timed",
     "ma_b200_device_status", "ma_b200_status_string", "ma_b200_last_error", "ma_b200_abi_version",
     "ma_b200_forward_static_scratch", "ma_b200_static_scratch_bytes", "ma_b200_static_scratch_last_error",
     "ma_b200_host_scratch_bytes", "ma_b200_forward_host", "ma_b200_forward_host_streamed", "ma_b200_host_last_error",
@@ -73,6 +73,8 @@ def load() -> C.CDLL:
     lib.ma_b200_workspace_bytes.restype = C.c_size_t
     lib.ma_b200_workspace_layout_of.argtypes = [pp, C.POINTER(WorkspaceLayout)]
     lib.ma_b200_workspace_layout_of.restype = C.c_int
+    lib.ma_b200_kernel_of_part.argtypes = [pp, C.c_int64]
+    lib.ma_b200_kernel_of_part.restype = C.c_int
     lib.ma_b200_forward.argtypes = [pp, C.c_void_p, C.c_size_t, C.c_void_p]
     lib.ma_b200_forward.restype = C.c_int
     lib.ma_b200_forward_timed.argtypes = [pp, C.c_void_p, C.c_size_t, C.c_void_p, C.POINTER(C.c_float), C.c_int32]

@@ -91,9 +91,8 @@ ma::Geometry make_geometry(const ma_b200_problem* p, int mask_type = MA_B200_MAS
 // sweep of blocks and counts of 16 to 200, 4 to 256 heads and widths 32 and 64: a tile takes 12.5 ns of the GPU's time and an
 // iteration 18.6 us at the least (8 beside the tiles' own time); a padded element of a warp-level tile takes 2.4 ps (1.7 in
 // heads of up to 32), two launches 6 us.
-bool warp_beats_tiles(const ma::Geometry& g) {
+bool warp_beats_tiles(const ma::Geometry& g, double heads) {
   if (g.B > 128 || g.M > 128) return false;  // (the warp-level kernels then walk a row twice: never the faster ones)
-  const double heads = (double)g.E * g.H;
   auto up16 = [](int x) { return (x + 15) & ~15; };
   auto keys = [](int x) { return x <= 16 ? 16 : x <= 32 ? 32 : x <= 64 ? 64 : 128; };
   const double elements = heads * ((double)g.M * up16(g.B) * keys(g.B) + (double)g.B * up16(g.M) * keys(g.M));
@@ -103,7 +102,9 @@ bool warp_beats_tiles(const ma::Geometry& g) {
   return warp_us < (tile_us > 18.6 ? tile_us : 18.6);
 }
 
-int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, int* kernel) {
+// AUTO goes by the shape of a head and by how many heads there are.  `heads`: the (batch, head) pairs of the whole call, of
+// which `p` may be a part: families differ in the order of their sums, so the parts of one call take the same one.
+int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, long long heads, int* kernel) {
   const char* why = "";
   const bool tc_ok = ma::tc_supported(g, p->qk_dtype, p->v_dtype, &why);
   const bool wants_tc = p->kernel == MA_B200_KERNEL_TCGEN05 || p->kernel == MA_B200_KERNEL_TCGEN05_STAGED;
@@ -135,16 +136,16 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, int* kernel)
   // The pipelined fused kernel takes a tile through a stage in 5 us, the tile kernels in 7 to 8, but those do 1.2 to 1.3
   // times as many tiles in a time: the fused kernel where a stage has no more tiles than fit the GPU at once (592; measured
   // at 512 tiles 41 against 43 us, at 1024 tiles 74 against 68), half as many when there is one iteration only.
-  const bool few_tiles = (long long)p->E * p->H * p->N / 128 * (p->num_steps == 1 ? 2 : 1) <= 592;
+  const bool few_tiles = heads * p->N / 128 * (p->num_steps == 1 ? 2 : 1) <= 592;
   // Head widths other than 64 and 72 have one tile size for both kinds of stage in the head-resident kernel: with one side of
   // up to 16 beside a longer one, and heads enough to fill the GPU, the warp-level kernels pad less (300 heads of 10 x 30 x 80:
   // 68 against 88 us).
-  const bool lopsided = (g.B <= 16) != (g.M <= 16) && g.D != 64 && g.D != 72 && (long long)p->E * p->H > 148;
+  const bool lopsided = (g.B <= 16) != (g.M <= 16) && g.D != 64 && g.D != 72 && heads > 148;
   if (p->kernel == MA_B200_KERNEL_AUTO)
     // (the older one-CTA-per-head kernel, HEAD_FUSED, is selectable but never preferred)
     *kernel = tc_ok && few_tiles ? MA_B200_KERNEL_TCGEN05
               : resident_ok && !lopsided ? MA_B200_KERNEL_HEAD_RESIDENT
-              : tile_ok && !(warp_ok && warp_beats_tiles(g)) ? MA_B200_KERNEL_TILE
+              : tile_ok && !(warp_ok && warp_beats_tiles(g, (double)heads)) ? MA_B200_KERNEL_TILE
               : warp_ok          ? MA_B200_KERNEL_WARP_MMA
               : tf32_pays        ? MA_B200_KERNEL_TF32X3
                                  : MA_B200_KERNEL_GENERIC;
@@ -164,7 +165,7 @@ int layout_of(const ma_b200_problem* p, ma_b200_workspace_layout* L) {
   if (rc != MA_B200_OK) return rc;
   ma::Geometry g = make_geometry(p);
   int kernel = 0;
-  rc = resolve_kernel(p, g, &kernel);
+  rc = resolve_kernel(p, g, (long long)p->E * p->H, &kernel);
   if (rc != MA_B200_OK) return rc;
   const size_t EH = (size_t)p->E * p->H, MB = (size_t)g.M * g.B;
   const size_t qs = dtype_size(p->qk_dtype), vs = dtype_size(p->v_dtype);
@@ -323,6 +324,16 @@ size_t ma_b200_workspace_bytes(const ma_b200_problem* p) {
 int ma_b200_workspace_layout_of(const ma_b200_problem* p, ma_b200_workspace_layout* layout) {
   if (layout == nullptr) return fail(MA_B200_INVALID_ARGUMENT, "layout is NULL");
   return layout_of(p, layout);
+}
+
+int ma_b200_kernel_of_part(const ma_b200_problem* part, int64_t heads) {
+  if (validate(part, false) != MA_B200_OK) return 0;
+  if (heads < (int64_t)part->E * part->H || heads > 0x7fffffffLL) {
+    fail(MA_B200_INVALID_ARGUMENT, "heads must count at least the part's own E*H, and fit 31 bits");
+    return 0;
+  }
+  int kernel = 0;
+  return resolve_kernel(part, make_geometry(part), heads, &kernel) == MA_B200_OK ? kernel : 0;
 }
 
 int ma_b200_forward(const ma_b200_problem* p, void* workspace, size_t workspace_bytes, void* stream) {

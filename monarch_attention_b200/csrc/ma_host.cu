@@ -5,7 +5,8 @@
 // independent in every stage, so the call is cut into chunks of a few heads and pipelined over
 // three streams owned by the library -
 //     copy-in : H2D q, k, v of chunk i+1
-//     compute : ma_b200_forward on chunk i (device staging buffers, E = 1, H = heads of the chunk)
+//     compute : ma_b200_forward on chunk i (device staging buffers, E = 1, H = heads of the chunk; the kernel family of
+//               the whole call, so that the result has the bits of one call on device tensors)
 //     copy-out: D2H result of chunk i-1
 // - with three staging slots in caller-provided device memory and events between the streams.
 // PCIe is full duplex, so the steady state is bound by the larger copy direction alone; the chunks of
@@ -202,7 +203,7 @@ static int forward_host_impl(const ma_b200_problem* p, int heads_per_chunk, void
     }
   }
 
-  int i = 0;
+  int i = 0, kernel = 0;  // one kernel family for all chunks: the one of a call on device tensors with all heads
   for (int e = 0; e < p->E; ++e) {
     int nh = 0;
     for (int h0 = 0; h0 < p->H; h0 += nh, ++i) {
@@ -235,6 +236,8 @@ static int forward_host_impl(const ma_b200_problem* p, int heads_per_chunk, void
       sub.out = {so, (int64_t)nh * p->N * p->Dv, (int64_t)p->N * p->Dv, p->Dv};
       sub.mask = mask_dev != nullptr ? mask_dev + (size_t)e * p->N : nullptr;
       sub.mask_stride_e = mask_dev != nullptr ? p->N : 0;
+      if (kernel == 0) kernel = ma_b200_kernel_of_part(&sub, (int64_t)p->E * p->H);
+      if (kernel != 0) sub.kernel = kernel;  // (0: ma_b200_forward says why)
       rc = ma_b200_forward(&sub, base + L.ws_off, L.ws_bytes, P->comp);
       if (rc != MA_B200_OK) {
         g_host_error = std::string("chunk forward: ") + ma_b200_last_error();

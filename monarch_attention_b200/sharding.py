@@ -4,7 +4,8 @@ Every (e, h) pair of a MonarchAttention call is independent in all four stages
 (reference: ma/ma_torch.py:65-108 has no reduction over E or H; the Triton grids are
 flat over E*H, ma/ma_triton.py:656-657), so the op shards across devices without any
 data-path collective: each rank runs the library on its own slice of the batch or
-head axis.  The only communication is a gather of per-rank timings and checksums
+head axis (with the kernel family of the whole call where the bits of the unsharded
+result are wanted: ``kernel_of_part``).  The only communication is a gather of per-rank timings and checksums
 for reporting.
 """
 from __future__ import annotations
@@ -43,6 +44,26 @@ def shard_heads(q, k, v, rank: int, world: int):
         return t.reshape(1, E * H, t.shape[2], t.shape[3])[:, lo:hi]
 
     return flat(q), flat(k), flat(v)
+
+
+def kernel_of_part(q, k, v, attn_mask, T: int, B: int, pre_pad: bool, heads: int) -> int:
+    """Kernel family of a call with ``heads`` (batch, head) pairs of which q, k, v are some.
+
+    The default choice goes by the number of heads in the call, and families differ in the last bits of the result.  A
+    rank that passes the answer on, ``monarch_attention_b200(..., kernel=kernel_of_part(...))``, computes the bits of the
+    unsharded call.
+    """
+    import ctypes as C
+
+    from . import _cabi
+    from .monarch_attention import make_problem
+
+    lib = _cabi.load()
+    q, k, v = (t if t.stride(-1) == 1 else t.contiguous() for t in (q, k, v))
+    kernel = lib.ma_b200_kernel_of_part(C.byref(make_problem(q, k, v, v, attn_mask, T, B, pre_pad)), heads)
+    if kernel == 0:
+        raise ValueError("monarch_attention_b200: " + lib.ma_b200_last_error().decode())
+    return kernel
 
 
 def gather_to_rank0(values, group=None):

@@ -120,6 +120,33 @@ def test_unit_range_partitions():
         unit_range(4, 4, 4)
 
 
+def test_parts_of_a_call_take_the_family_of_the_whole_call(lib):
+    """AUTO goes by the number of heads (here: one side of up to 16 beside a longer one, and heads enough to fill the GPU);
+    a part that names the whole call's heads gets the whole call's family."""
+    from monarch_attention_b200 import _cabi
+    shape = dict(N=300, D=80, Dv=80, block_size=10, qk_dtype=_cabi.BF16, v_dtype=_cabi.BF16)
+    whole, part = _problem(E=30, H=20, **shape), _problem(E=1, H=8, **shape)
+    L = _cabi.WorkspaceLayout()
+
+    def auto(p):
+        _cabi.raise_for_status(lib.ma_b200_workspace_layout_of(C.byref(p), C.byref(L)))
+        return L.kernel
+
+    assert auto(whole) != auto(part)
+    assert lib.ma_b200_kernel_of_part(C.byref(part), 600) == lib.ma_b200_kernel_of_part(C.byref(whole), 600) == auto(whole)
+    assert lib.ma_b200_kernel_of_part(C.byref(part), 8) == auto(part)
+    pinned = _problem(E=1, H=8, kernel=_cabi.KERNEL_GENERIC, **shape)
+    assert lib.ma_b200_kernel_of_part(C.byref(pinned), 600) == _cabi.KERNEL_GENERIC
+    assert lib.ma_b200_kernel_of_part(C.byref(part), 7) == 0 and b"heads" in lib.ma_b200_last_error()
+    assert lib.ma_b200_kernel_of_part(C.byref(_problem(E=0)), 600) == 0
+    assert lib.ma_b200_kernel_of_part(None, 600) == 0
+    from monarch_attention_b200.sharding import kernel_of_part
+    q = torch.zeros(1, 8, 300, 80, dtype=torch.bfloat16)
+    assert kernel_of_part(q, q, q, None, 2, 10, False, 600) == auto(whole)
+    with pytest.raises(ValueError):
+        kernel_of_part(q, q, q, None, 2, 10, False, 1)
+
+
 _WORKER = r"""
 import os, sys
 sys.path.insert(0, {root!r}); sys.path.insert(0, os.path.join({root!r}, "tests", "golden"))
