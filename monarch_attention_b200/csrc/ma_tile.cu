@@ -62,7 +62,8 @@ enum {
   kBarO = 7,     // O in tensor memory
   kBarE = 8,     // O read and staged in shared memory by the 128 row threads
   kBarFree = 9,  // staging tile read by the store
-  kTileBars = 10
+  kBarDrain = 10,  // after a wait that gave up: the tensor pipe has finished
+  kTileBars = 11
 };
 constexpr int kRowBarrier = 1;  // named barrier of the row threads
 constexpr int kTileThreads = kRows + 32;
@@ -304,9 +305,13 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(NK))
       if (lane == 0) {
         give_up(701);
         // own copies have landed before the CTA leaves
-        for (int i = la > 2 ? la - 2 : 0; i < la; ++i) (void)mbar_wait(bar(kBarA + (kTwoA ? i & 1 : 0)), (uint32_t)(kTwoA ? i >> 1 : i) & 1u);
-        for (int i = lb > 2 ? lb - 2 : 0; i < lb; ++i) (void)mbar_wait(bar(kBarB + (kTwoB ? i & 1 : 0)), (uint32_t)(kTwoB ? i >> 1 : i) & 1u);
+        constexpr int na = kTwoA ? 2 : 1, nb = kTwoB ? 2 : 1;  // (one slot has one load in flight)
+        for (int i = max(la - na, 0); i < la; ++i) (void)mbar_wait(bar(kBarA + (kTwoA ? i & 1 : 0)), (uint32_t)(kTwoA ? i >> 1 : i) & 1u);
+        for (int i = max(lb - nb, 0); i < lb; ++i) (void)mbar_wait(bar(kBarB + (kTwoB ? i & 1 : 0)), (uint32_t)(kTwoB ? i >> 1 : i) & 1u);
         if (lv > 0) (void)mbar_wait(bar(kBarV), (uint32_t)(lv - 1) & 1u);
+        // the contractions that were issued have read their operands and written tensor memory
+        mma_commit(bar(kBarDrain));
+        (void)mbar_wait(bar(kBarDrain), 0);
       }
     } else if (my_tiles > 0) {
       store(KIND == kStageRightWithV ? &maps.s1 : &maps.s0, my_tiles - 1, (kChunks - 1) * kRows);
