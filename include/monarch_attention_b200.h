@@ -185,9 +185,9 @@ MA_B200_API int ma_b200_backward_typed_mask(const ma_b200_problem* p, int mask_t
  * this workspace: MA_B200_OK or MA_B200_DEVICE_WAIT_EXPIRED. */
 MA_B200_API int ma_b200_device_status(void* workspace, void* stream);
 
-/* Without synchronising anything: has a bounded wait of the fused tcgen05 kernel given up on `device`
+/* Without synchronising anything: has a bounded wait of a tcgen05 kernel given up on `device`
  * since the last poll?  A CTA that gives up stores its code in a page-locked host word the library
- * maps once per device (at the first fused launch there), so the answer trails the GPU by at most
+ * maps once per device (at the first launch of such a kernel), so the answer trails the GPU by at most
  * the kernels still in flight.  MA_B200_OK, or MA_B200_DEVICE_WAIT_EXPIRED once per incident (the
  * word is cleared by the poll).  This is the lazily read error flag of the eager call: the reference
  * raises from inside the call (ma/monarch_attention.py:50-59), an asynchronous launch cannot.
@@ -197,7 +197,9 @@ MA_B200_API int ma_b200_poll_device_status(int device);
 /* Self-test of the give-up path (no counterpart in the reference): launches the left-factor stage of
  * `p` (num_steps >= 2, a problem the fused kernel takes) alone, with the completion counters it waits
  * on left at zero and a short patience, so that every CTA's bounded wait runs out and the kernel
- * returns by itself after a few hundred microseconds.  Afterwards ma_b200_device_status(workspace)
+ * returns by itself after a few hundred microseconds.  With p->kernel = MA_B200_KERNEL_TILE the same for the tile
+ * kernels: the single launch without its first stage, or (block size or count above 128) the first stage's kernel with
+ * an operand that is never asked for.  Afterwards ma_b200_device_status(workspace)
  * and ma_b200_poll_device_status() report MA_B200_DEVICE_WAIT_EXPIRED, and the next ordinary call is
  * unaffected.  Nothing faults, traps or spins without bound. */
 MA_B200_API int ma_b200_selftest_wait_expiry(const ma_b200_problem* p, void* workspace, size_t workspace_bytes,

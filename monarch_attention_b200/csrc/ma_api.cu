@@ -257,9 +257,9 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
   auto launch = [&](ma::StageKind kind, bool first) -> cudaError_t {
     cudaError_t e;
     if (L.kernel == MA_B200_KERNEL_TCGEN05_STAGED)
-      e = ma::launch_fused(plan, g, counters, stage_idx, stage_idx + 1, 0, stream);
+      e = ma::launch_fused(plan, g, counters, stage_idx, stage_idx + 1, 0, 0, stream);
     else if (L.kernel == MA_B200_KERNEL_TILE)
-      e = ma::launch_tile_stage(g, p->qk_dtype, kind, first, host_status, stream);
+      e = ma::launch_tile_stage(g, p->qk_dtype, kind, first, host_status, false, stream);
     else if (L.kernel == MA_B200_KERNEL_WARP_MMA || L.kernel == MA_B200_KERNEL_TF32X3)
       e = ma::launch_warp_stage(g, p->qk_dtype, kind, first, stream);
     else e = ma::launch_generic_stage(g, p->qk_dtype, p->v_dtype, kind, first, stream);
@@ -277,11 +277,11 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
     if (ev != nullptr)
       for (int i = 1; i <= n_stages; ++i) cudaEventRecord(ev[i], stream);
   } else if (flow) {
-    ce = ma::launch_flow(g, p->qk_dtype, counters, host_status, stream);
+    ce = ma::launch_flow(g, p->qk_dtype, counters, host_status, false, stream);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "tile kernels in one launch");
   } else if (L.kernel == MA_B200_KERNEL_TCGEN05) {
     // every stage in one persistent launch
-    ce = ma::launch_fused(plan, g, counters, 0, n_stages, 1, stream);
+    ce = ma::launch_fused(plan, g, counters, 0, n_stages, 1, 0, stream);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "fused kernel");
     if (ev != nullptr) {
       cudaEventRecord(ev[1], stream);
@@ -417,7 +417,7 @@ int ma_b200_poll_device_status(int device) {
   const int code = ma::fused_poll_status(device);
   if (code != 0)
     return fail(MA_B200_DEVICE_WAIT_EXPIRED, "device " + std::to_string(device) + ": wait " + std::to_string(code) +
-                                                 " of the fused kernel gave up; the output of that call is undefined");
+                                                 " of a kernel gave up; the output of that call is undefined");
   return MA_B200_OK;
 }
 
@@ -427,7 +427,7 @@ int ma_b200_selftest_wait_expiry(const ma_b200_problem* p, void* workspace, size
   int rc = validate(p, true);
   if (rc != MA_B200_OK) return rc;
   ma_b200_problem q = *p;
-  q.kernel = MA_B200_KERNEL_TCGEN05;
+  if (q.kernel != MA_B200_KERNEL_TILE) q.kernel = MA_B200_KERNEL_TCGEN05;
   ma_b200_workspace_layout L;
   rc = layout_of(&q, &L);
   if (rc != MA_B200_OK) return rc;
@@ -442,15 +442,25 @@ int ma_b200_selftest_wait_expiry(const ma_b200_problem* p, void* workspace, size
   g.y = ws + L.y;
   cudaError_t ce = cudaMemsetAsync(ws + L.status, 0, L.ar - L.status, stream);
   if (ce != cudaSuccess) return fail(MA_B200_CUDA_ERROR, cudaGetErrorString(ce));
+  if (q.kernel == MA_B200_KERNEL_TILE) {
+    int dev = 0;
+    if ((ce = cudaGetDevice(&dev)) != cudaSuccess) return fail(MA_B200_CUDA_ERROR, cudaGetErrorString(ce));
+    int* const host_status = ma::host_status_word(dev);
+    // The single launch: its first stage is left out, and every CTA waits for that.  The kernels of a launch each: the
+    // first stage, with an operand that no CTA asks for.
+    ce = ma::flow_supported(g) ? ma::launch_flow(g, q.qk_dtype, reinterpret_cast<int*>(ws + L.counters), host_status, true, stream)
+                               : ma::launch_tile_stage(g, q.qk_dtype, q.num_steps > 1 ? ma::kStageRight : ma::kStageRightWithV, true,
+                                                       host_status, true, stream);
+    if (ce != cudaSuccess) return fail(MA_B200_CUDA_ERROR, std::string("tile kernels: ") + cudaGetErrorString(ce));
+    return MA_B200_OK;
+  }
   ma::TcPlan plan;
   const char* err = "";
   rc = ma::tc_plan_get(g, q.qk_dtype, &plan, &err);
   if (rc != MA_B200_OK) return fail(rc, std::string("tcgen05 plan: ") + err);
   // Stage 1 alone, waiting on completion counters of stage 0 that nothing will ever raise: every
   // producer runs out of patience after a few hundred microseconds and the CTAs return.
-  ma::fused_set_spin_limit(4096);
-  ce = ma::launch_fused(&plan, g, reinterpret_cast<int*>(ws + L.counters), 1, 2, 1, stream);
-  ma::fused_set_spin_limit(0);
+  ce = ma::launch_fused(&plan, g, reinterpret_cast<int*>(ws + L.counters), 1, 2, 1, 4096, stream);
   if (ce != cudaSuccess) return fail(MA_B200_CUDA_ERROR, std::string("fused kernel: ") + cudaGetErrorString(ce));
   return MA_B200_OK;
 }

@@ -167,21 +167,21 @@ int tc_plan_create(const Geometry& g, int qk_dtype, TcPlan** plan, const char** 
 void tc_plan_destroy(TcPlan* plan);
 // Persistent fused kernel: stages [stage_begin, stage_end) of the 2T stages in one cooperative launch.
 size_t fused_counter_bytes(const Geometry& g);
+// (spin_limit: iterations of the dependency wait before it gives up, 0 = default; for the wait-expiry self-test.)
 cudaError_t launch_fused(const TcPlan* plan, const Geometry& g, int* counters, int stage_begin, int stage_end,
-                         int wait_deps, cudaStream_t stream);
+                         int wait_deps, int spin_limit, cudaStream_t stream);
 // Device address of the mapped host word that a kernel whose bounded wait gave up stores its code in (nullptr: none).
 int* host_status_word(int device);
 // tcgen05 stage kernels, one 128-row tile per CTA: block size and count up to 256, D <= 64, masks and padding (ma_tile.cu).
 bool tile_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
-cudaError_t launch_tile_stage(const Geometry& g, int dtype, StageKind kind, bool first, int* host_status, cudaStream_t stream);
+// wait_expiry (self-test): a wait of every CTA runs out.
+cudaError_t launch_tile_stage(const Geometry& g, int dtype, StageKind kind, bool first, int* host_status, bool wait_expiry, cudaStream_t stream);
 // Their single-launch form, all stages of a call, for block size and count up to 128 (ma_flow.cu); counters: (E*H, 2T)
-// zeroed ints.
+// zeroed ints, as the status block.  wait_expiry (self-test): the first stage is left out, so that the waits for it run out.
 bool flow_supported(const Geometry& g);
-cudaError_t launch_flow(const Geometry& g, int dtype, int* counters, int* host_status, cudaStream_t stream);
+cudaError_t launch_flow(const Geometry& g, int dtype, int* counters, int* host_status, bool wait_expiry, cudaStream_t stream);
 // Code of a bounded device-side wait that gave up on `device` since the last poll (0 = none); reads a mapped
 // host word, so it needs no synchronisation.
 int fused_poll_status(int device);
-// Iterations of the producer's dependency wait before it gives up (0 = default); for the wait-expiry self-test.
-void fused_set_spin_limit(int iterations);
 
 }  // namespace ma

@@ -896,12 +896,9 @@ int* host_status_word(int device) {
   return hs.dev;
 }
 
-static int g_spin_limit_override = 0;
-void fused_set_spin_limit(int iterations) { g_spin_limit_override = iterations; }
-
 // Runs stages [stage_begin, stage_end) in one cooperative launch.
 cudaError_t launch_fused(const TcPlan* plan, const Geometry& g, int* counters, int stage_begin, int stage_end,
-                         int wait_deps, cudaStream_t stream) {
+                         int wait_deps, int spin_limit, cudaStream_t stream) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -946,7 +943,7 @@ cudaError_t launch_fused(const TcPlan* plan, const Geometry& g, int* counters, i
   }
   a.wait_deps = wait_deps;
   a.reuse_slots = wait_deps && (stage_begin == 0 && stage_end == 2 * g.T) ? 1 : 0;
-  a.spin_limit = g_spin_limit_override > 0 ? g_spin_limit_override : (1 << 24);
+  a.spin_limit = spin_limit > 0 ? spin_limit : (1 << 24);
   a.counters = counters;
   a.host_status = host_status_dev;
   const int total = (stage_end - stage_begin) * (g.N / kTile) * g.E * g.H;

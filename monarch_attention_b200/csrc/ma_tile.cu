@@ -32,6 +32,7 @@ struct TileArgs {
   int tiles, total;  // tiles per head, and of all heads
   int first;         // right-factor: first iteration (A = q, cr = 1)
   int clear;         // this launch clears the status word
+  int hold;          // self-test: the first operand of a CTA is never asked for; tries until the wait for it gives up
   int* host_status;  // mapped host word for a wait that gave up, or nullptr
 };
 
@@ -232,14 +233,14 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(NK))
       mbar_arrive(bar(kBarFree));
     };
 
-    load_a(0);
+    if (args.hold == 0) load_a(0);
     load_b(0);
     load_v(0);
     if (kTwoA) load_a(1);
     if (kTwoB) load_b(1);
     uint32_t ns = 0, np = 0, no = 0, ne = 0;  // phases of S, P, O, E waited for
-    bool ok = true;
-    for (int i = 0; i < my_tiles; ++i) {
+    bool ok = args.hold == 0 || __all_sync(0xffffffffu, mbar_wait_abortable(bar(kBarA), 0, abort_flag, args.hold));
+    for (int i = 0; ok && i < my_tiles; ++i) {
       ok = wait(kBarA + (kTwoA ? i & 1 : 0), kTwoA ? i >> 1 : i) && wait(kBarB + (kTwoB ? i & 1 : 0), kTwoB ? i >> 1 : i);
       if (!ok) break;
       if (!kRight && g.N != whole * B) {  // the token of the row behind the last whole one (its place was zero-filled)
@@ -306,7 +307,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(NK))
         give_up(701);
         // own copies have landed before the CTA leaves
         constexpr int na = kTwoA ? 2 : 1, nb = kTwoB ? 2 : 1;  // (one slot has one load in flight)
-        for (int i = max(la - na, 0); i < la; ++i) (void)mbar_wait(bar(kBarA + (kTwoA ? i & 1 : 0)), (uint32_t)(kTwoA ? i >> 1 : i) & 1u);
+        for (int i = max(la - na, args.hold != 0 ? 1 : 0); i < la; ++i) (void)mbar_wait(bar(kBarA + (kTwoA ? i & 1 : 0)), (uint32_t)(kTwoA ? i >> 1 : i) & 1u);
         for (int i = max(lb - nb, 0); i < lb; ++i) (void)mbar_wait(bar(kBarB + (kTwoB ? i & 1 : 0)), (uint32_t)(kTwoB ? i >> 1 : i) & 1u);
         if (lv > 0) (void)mbar_wait(bar(kBarV), (uint32_t)(lv - 1) & 1u);
         // the contractions that were issued have read their operands and written tensor memory
@@ -584,7 +585,7 @@ cudaError_t launch_tile_kind(const Geometry& g, StageKind kind, const TileMaps& 
 }
 
 template <typename T>
-cudaError_t launch_tile_dtype(const Geometry& g, int dtype, StageKind kind, bool first, int* host_status, cudaStream_t stream) {
+cudaError_t launch_tile_dtype(const Geometry& g, int dtype, StageKind kind, bool first, int* host_status, bool wait_expiry, cudaStream_t stream) {
   const bool right = is_right(kind);
   const int keys = right ? g.B : g.M, nk = keys <= 64 ? 64 : keys <= 128 ? 128 : 256;
   const int a_rows = nk == 64 ? 64 : nk == 256 && kind == kStageLeft ? 256 : 128, b_rows = nk, s_rows = nk == 64 ? 64 : 128;
@@ -608,6 +609,7 @@ cudaError_t launch_tile_dtype(const Geometry& g, int dtype, StageKind kind, bool
   TileArgs args{};
   args.first = first ? 1 : 0;
   args.clear = right && first ? 1 : 0;
+  args.hold = wait_expiry ? 4096 : 0;
   args.host_status = host_status;
   if (nk == 64) return launch_tile_kind<T, 64>(g, kind, maps, args, stream);
   if (nk == 128) return launch_tile_kind<T, 128>(g, kind, maps, args, stream);
@@ -639,9 +641,9 @@ bool tile_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** w
   return true;
 }
 
-cudaError_t launch_tile_stage(const Geometry& g, int dtype, StageKind kind, bool first, int* host_status, cudaStream_t stream) {
-  if (dtype == MA_B200_BF16) return launch_tile_dtype<__nv_bfloat16>(g, dtype, kind, first, host_status, stream);
-  return launch_tile_dtype<__half>(g, dtype, kind, first, host_status, stream);
+cudaError_t launch_tile_stage(const Geometry& g, int dtype, StageKind kind, bool first, int* host_status, bool wait_expiry, cudaStream_t stream) {
+  if (dtype == MA_B200_BF16) return launch_tile_dtype<__nv_bfloat16>(g, dtype, kind, first, host_status, wait_expiry, stream);
+  return launch_tile_dtype<__half>(g, dtype, kind, first, host_status, wait_expiry, stream);
 }
 
 }  // namespace ma

@@ -1,6 +1,8 @@
 """tcgen05 tile kernels at the edges of their tiles (two units per tile with an odd last one, row and column remainders,
 the row behind the last whole block, both padding sides, masks that empty blocks, narrow heads, several tiles per CTA),
 against the CPU oracle."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -60,3 +62,36 @@ def test_single_launch_stages_read_what_the_stage_before_wrote(H, B, M, T):
     for _ in range(10):
         for x, w in zip(inputs, want):
             assert torch.equal(mod(*x), w)
+
+
+@pytest.mark.parametrize("E,H,N,B,T", [(1, 2, 4096, 64, 2), (2, 12, 4096, 64, 1), (1, 3, 128 * 100 - 5, 128, 3),
+                                       (1, 2, 40 * 100, 40, 2), (1, 2, 200 * 40, 200, 2), (1, 1, 256 * 256, 256, 1)])
+def test_expired_wait_ends_the_launch_and_is_reported(E, H, N, B, T):
+    """Single launch: the first stage is left out, so the waits for it run out; one launch per stage (blocks above 128): an
+    operand is never asked for.  Every CTA gives up by itself, the status words say so, the next call raises, and the one
+    after is an ordinary call."""
+    import monarch_attention_b200 as ma
+    from monarch_attention_b200 import _cabi
+    from monarch_attention_b200.monarch_attention import make_problem
+    lib, dev = _cabi.load(), torch.device("cuda:0")
+    g = torch.Generator().manual_seed(N)
+    q, k, v = (torch.randn(E, H, N, 64, generator=g).to(torch.bfloat16).to(dev) for _ in range(3))
+    mod = ma.MonarchAttention(B, T, "post", impl="b200-tile")
+    good = mod(q, k, v)
+    stream = torch.cuda.current_stream().cuda_stream
+    prob = make_problem(q, k, v, torch.empty_like(v), None, T, B, False, _cabi.KERNEL_TILE)
+    ws = torch.zeros(lib.ma_b200_workspace_bytes(C.byref(prob)), dtype=torch.uint8, device=dev)
+    assert lib.ma_b200_poll_device_status(0) == _cabi.OK
+    start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    start.record()
+    _cabi.raise_for_status(lib.ma_b200_selftest_wait_expiry(C.byref(prob), ws.data_ptr(), ws.numel(), stream))
+    end.record()
+    torch.cuda.synchronize()
+    # the waits that run out are of 4096 tries; what a CTA still waits for on its way out has been asked for and is there
+    # (a wait for something else would be one of millions of tries)
+    assert start.elapsed_time(end) < 500
+    assert lib.ma_b200_device_status(ws.data_ptr(), stream) == _cabi.DEVICE_WAIT_EXPIRED
+    with pytest.raises(RuntimeError, match="gave up"):
+        mod(q, k, v)
+    assert lib.ma_b200_poll_device_status(0) == _cabi.OK
+    assert torch.equal(mod(q, k, v), good)
