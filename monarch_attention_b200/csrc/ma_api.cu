@@ -133,17 +133,22 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, long long he
   // Heads narrower than 24 leave most of a 16-wide contraction step of the fp32 tensor path padded or give it one
   // step per tile; the thread-per-logit kernels are as fast there.
   const bool tf32_pays = tf32_ok && g.D >= 24;
-  // The pipelined fused kernel takes a tile through a stage in 5 us, the tile kernels in 7 to 8, but those do 1.2 to 1.3
-  // times as many tiles in a time: the fused kernel where a stage has no more tiles than fit the GPU at once (592; measured
-  // at 512 tiles 41 against 43 us, at 1024 tiles 74 against 68), half as many when there is one iteration only.
-  const bool few_tiles = heads * p->N / 128 * (p->num_steps == 1 ? 2 : 1) <= 592;
+  // The fused kernel takes one tile at a time through an SM, quickly; the tile kernels take four, each more slowly, and do
+  // 1.2 to 1.4 times as many in a time.  So the fused kernel is the faster one while a stage is few rounds of one tile per
+  // SM.  Measured (us, fused / tile kernels) over 32 to 2048 tiles per stage, blocks of 64 and 128: with two iterations 42 / 45 at
+  // 3.5 tiles per SM, 50 / 54 and 59 / 63 at 5.2, 54.8 / 55.8 at 5.8, 56.9 / 56.2 at 6.1, 77 / 59 and 75 / 68 at 6.9; with three
+  // 70 / 73 and 83 / 91 at 5.2, 75.2 / 74.1 at 5.8, 79 / 75 at 6.1: the line is at 5.5.  With one, whose two stages leave the tile
+  // kernels' list fewer waits, 20.7 / 20.7 and 21.5 / 22.8 at 1.7, 23.1 / 22.8 and 26.6 / 25.0 at 2.6: at 2.
+  const bool few_tiles = tc_ok && heads * p->N / 64 <= (long long)ma::sm_count() * (p->num_steps == 1 ? 4 : 11);
   // Head widths other than 64 and 72 have one tile size for both kinds of stage in the head-resident kernel: with one side of
-  // up to 16 beside a longer one, and heads enough to fill the GPU, the warp-level kernels pad less (300 heads of 10 x 30 x 80:
-  // 68 against 88 us).
-  const bool lopsided = (g.B <= 16) != (g.M <= 16) && g.D != 64 && g.D != 72 && heads > 148;
+  // up to 16 beside a longer one the warp-level kernels pad less, and win once the heads no longer fit the SMs in one round.
+  // Measured (us, head-resident / warp-level; widths 32 to 80, blocks of 8 x 20 to 16 x 24, one and two iterations), 10 x 30 x 80
+  // with two: 33 / 37 at 148 heads, 60 / 39 at 160, 88 / 62 at 300, 124 / 115 at 592; 10 x 30 x 32 with one: 13 / 16, 21 / 17,
+  // 32 / 23, 39 / 37.  (Against the rule: width 32 and many heads with two iterations, 61 / 78 at 592 heads of 16 x 24.)
+  const bool lopsided = (g.B <= 16) != (g.M <= 16) && g.D != 64 && g.D != 72 && heads > ma::sm_count();
   if (p->kernel == MA_B200_KERNEL_AUTO)
     // (the older one-CTA-per-head kernel, HEAD_FUSED, is selectable but never preferred)
-    *kernel = tc_ok && few_tiles ? MA_B200_KERNEL_TCGEN05
+    *kernel = few_tiles ? MA_B200_KERNEL_TCGEN05
               : resident_ok && !lopsided ? MA_B200_KERNEL_HEAD_RESIDENT
               : tile_ok && !(warp_ok && warp_beats_tiles(g, (double)heads)) ? MA_B200_KERNEL_TILE
               : warp_ok          ? MA_B200_KERNEL_WARP_MMA

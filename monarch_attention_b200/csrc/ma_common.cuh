@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -85,6 +86,17 @@ inline cudaError_t allow_dynamic_smem(const void* fn, size_t bytes) {
   e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e == cudaSuccess) have = bytes;
   return e;
+}
+
+// Multiprocessors of the current device (where there is none, as in a layout query: those of a B200).
+inline int sm_count() {
+  static std::atomic<int> counts[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if ((n = counts[dev].load(std::memory_order_relaxed)) == 0 &&
+      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+    counts[dev].store(n, std::memory_order_relaxed);
+  return n > 0 ? n : 148;
 }
 
 // Whether the mask lets token n of batch element e through.  The callers' masks come as booleans, integers or floats

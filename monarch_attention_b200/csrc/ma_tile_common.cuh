@@ -298,13 +298,5 @@ bool strided_state_map(CUtensorMap* m, int dtype, const Geometry& g, const void*
   return make_map(m, dtype, base, 4, dims, str, box);
 }
 
-int sm_count() {
-  static int counts[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (counts[dev] == 0) cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev);
-  return counts[dev] > 0 ? counts[dev] : 148;
-}
-
 }  // namespace
 }  // namespace ma
