@@ -275,8 +275,18 @@ constexpr size_t right_elems(bool with_v, int RP) {
   return (size_t)(2 * RP + KP + (with_v ? KP + RP : 0)) * (DP + 8) + (size_t)2 * RP * (KP + 8) + (size_t)kF<T> * KP;
 }
 
+// CTAs per SM that the 16-bit instances for up to 32 keys (the fine-tuning shapes) are compiled for: without V ten, at 96
+// registers; with V seven, which is what shared memory holds at width 64 (28.3 KB each), so that no register is given up for more.
+// 8 x 16 heads of 1024 tokens at width 72, two iterations: 334.7 us with ten for both kinds (the instances with V then
+// spill at widths above 64), 332.2 left to the compiler, 331.4 as it is; 4 x 12 heads at width 64, three iterations: 193.0, 193.7, 192.0.
+// The fp32 instances for up to 64 keys take all 255 registers and spill (460 bytes a thread at width 64, 776 with V; 860 and
+// 1076 at width 80): the logit and factor rows of a warp alone are 2 x 32 registers, their split halves as many again.  They are
+// still worth having: forward and backward of 2 x 12 heads of 4096 tokens, two iterations, 1074 us against 3425 by tensor
+// operations at width 64, 1605 against 4009 at width 80.
+constexpr int right_ctas(int element_bytes, int KP, bool with_v) { return KP == 32 && element_bytes == 2 ? (with_v ? 7 : 10) : 1; }
+
 template <typename T, int KP, int DP, bool WITH_V>
-__global__ void __launch_bounds__(2 * KP, KP == 32 && sizeof(T) == 2 ? 10 : 1) backward_right_kernel(const BackwardArgs a) {
+__global__ void __launch_bounds__(2 * KP, right_ctas(sizeof(T), KP, WITH_V)) backward_right_kernel(const BackwardArgs a) {
   constexpr int PITCH = DP + 8, PP = KP + 8;
   stage_begin();
   extern __shared__ __align__(16) uint8_t smem[];
