@@ -147,7 +147,6 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, long long he
   // 32 / 23, 39 / 37.  (Against the rule: width 32 and many heads with two iterations, 61 / 78 at 592 heads of 16 x 24.)
   const bool lopsided = (g.B <= 16) != (g.M <= 16) && g.D != 64 && g.D != 72 && heads > ma::sm_count();
   if (p->kernel == MA_B200_KERNEL_AUTO)
-    // (the older one-CTA-per-head kernel, HEAD_FUSED, is selectable but never preferred)
     *kernel = few_tiles ? MA_B200_KERNEL_TCGEN05
               : resident_ok && !lopsided ? MA_B200_KERNEL_HEAD_RESIDENT
               : tile_ok && !(warp_ok && warp_beats_tiles(g, (double)heads)) ? MA_B200_KERNEL_TILE
@@ -229,7 +228,7 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
   // (with per-stage times wanted, the tile kernels run one launch per stage)
   const bool flow = L.kernel == MA_B200_KERNEL_TILE && stage_ms == nullptr && ma::flow_supported(g);
   if (flow || (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3 && L.kernel != MA_B200_KERNEL_HEAD_RESIDENT &&
-               L.kernel != MA_B200_KERNEL_TILE)) {
+               L.kernel != MA_B200_KERNEL_HEAD_FUSED && L.kernel != MA_B200_KERNEL_TILE)) {
     ce = cudaMemsetAsync(ws + L.status, 0, L.ar - L.status, stream);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(status, counters)");
   }
@@ -276,9 +275,8 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
   rc = MA_B200_OK;
   bool first = true;
   if (L.kernel == MA_B200_KERNEL_HEAD_FUSED || L.kernel == MA_B200_KERNEL_HEAD_RESIDENT) {
-    ce = L.kernel == MA_B200_KERNEL_HEAD_FUSED ? ma::launch_head_fused(g, p->qk_dtype, stream)
-                                               : ma::launch_head_resident(g, p->qk_dtype, stream);
-    if (ce != cudaSuccess) rc = cuda_fail(ce, "one-CTA-per-head kernel");
+    ce = ma::launch_head_resident(g, p->qk_dtype, stream);
+    if (ce != cudaSuccess) rc = cuda_fail(ce, "head-resident kernel");
     if (ev != nullptr)
       for (int i = 1; i <= n_stages; ++i) cudaEventRecord(ev[i], stream);
   } else if (flow) {

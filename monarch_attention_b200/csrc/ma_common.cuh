@@ -151,9 +151,6 @@ bool warp_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** w
 // The same kernels on fp32 tensors (products of split operands on the tf32 tensor path).
 bool tf32x3_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
 cudaError_t launch_warp_stage(const Geometry& g, int qk_dtype, StageKind kind, bool first, cudaStream_t stream);
-// Whole head per CTA, both stages of a one-iteration call in one launch (state in shared memory).
-bool head_fused_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
-cudaError_t launch_head_fused(const Geometry& g, int qk_dtype, cudaStream_t stream);
 
 // Backward pass (ma_backward.cu): byte offsets in its workspace; al, ar, cl, cr hold one entry per iteration.
 struct BackwardLayout {
@@ -168,6 +165,8 @@ cudaError_t launch_backward(const Geometry& g, int dtype, const View4& dz, const
 // Head-resident kernel: all stages of a head in one launch, block size and count up to 32 (ma_head.cu).
 bool head_resident_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
 cudaError_t launch_head_resident(const Geometry& g, int qk_dtype, cudaStream_t stream);
+// The same kernel under the narrower limits of the HEAD_FUSED family.
+bool head_fused_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);
 
 // Tensor-core (tcgen05) path.
 bool tc_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why);

@@ -149,9 +149,9 @@ class MonarchAttention(nn.Module):
     problem fits it, otherwise the generic path), "b200-generic", "b200-tcgen05" (fused, one
     launch), "b200-tcgen05-staged" (same kernel, one launch per stage),
     "b200-warp-mma" (warp-level tensor-core kernels for small blocks),
-    "b200-head-fused" (one CTA per head, one iteration, state in shared memory), "b200-tf32x3"
-    (the warp-level kernels on fp32 tensors), "b200-head-resident" (one CTA or cluster per head, all stages) or
-    "b200-tile" (tcgen05 stage kernels, one 128-row tile per CTA).  The reference's
+    "b200-tf32x3" (the same on fp32 tensors), "b200-head-resident" (one CTA or cluster per head, all
+    stages), "b200-head-fused" (the same, one iteration only) or "b200-tile" (tcgen05 tile kernels, one launch
+    up to blocks of 128).  The reference's
     "torch" and "triton" implementations are not part of this library; asking for an
     unknown name raises ``ValueError`` exactly as the reference does.
     """
