@@ -339,12 +339,15 @@ def time_reference_gpu(q, k, v, T, B, reps=5):
     return out
 
 
-def fused_kernel_dram_traffic():
-    """dram__bytes_read.sum + dram__bytes_write.sum of one launch of the fused kernel on the headline workload,
-    as recorded in the committed ncu summary (a profiler cannot run inside this script)."""
+def dram_traffic(kernel_name):
+    """dram__bytes_read.sum + dram__bytes_write.sum of one launch on the headline workload, as recorded in the committed
+    ncu summary of the kernel that runs it (a profiler cannot run inside this script)."""
     import re
+    summary = {"tcgen05-fused": "fused_kernel_c3_n16384_bf16.md", "tile": "tile_flow_kernel_c3_n16384_bf16.md"}.get(kernel_name)
+    if summary is None:
+        return None
     try:
-        text = open(os.path.join(ROOT, "profiles", "fused_kernel_c3_n16384_bf16.md")).read()
+        text = open(os.path.join(ROOT, "profiles", summary)).read()
         m = re.search(r"dram_traffic_bytes_per_launch\s*=\s*([0-9.eE+]+)", text)
         return float(m.group(1)) if m else None
     except OSError:
@@ -489,7 +492,7 @@ def run_ours(args, rank, world, local):
         return
 
     # ---- per-stage launch durations (CUDA events on the launching stream, inside the library) ------
-    # (the headline runs all stages in one launch; the stages launched one by one give the breakdown)
+    # (the headline runs all stages in one launch; the fused kernel can launch them one by one, which gives a breakdown)
     q, k, v = sets[0]
     staged = _cabi.KERNEL_TCGEN05_STAGED if kernel == _cabi.KERNEL_TCGEN05 else kernel
     prob = make_problem(q, k, v, outs[0], None, w["T"], w["B"], False, staged)
@@ -514,24 +517,25 @@ def run_ours(args, rank, world, local):
     if strong:
         flops, nbytes = flops / world, nbytes / world  # this rank's share; the roofline below is per GPU
     names = ["right", "left", "right_with_v", "output"]
+    if kernel == _cabi.KERNEL_TILE:
+        names, stage_flops = ["all_in_one_launch"], {"all_in_one_launch": sum(stage_flops.values())}
     stages = [{"stage": n, "ms": acc[i], "tflops": stage_flops[n] / (world if strong else 1) / (acc[i] * 1e-3) / 1e12}
               for i, n in enumerate(names)]
     peaks = measured_peaks()
     t_tensor = flops / (peaks["bf16_tflops"] * 1e12)
     t_hbm = nbytes / (peaks["hbm_gbs"] * 1e9)
     achieved_tflops = flops / (ms_step * 1e-3) / 1e12
-    fused = kernel == _cabi.KERNEL_TCGEN05
     one_launch = kernel in (_cabi.KERNEL_TCGEN05, _cabi.KERNEL_TILE)
     roofline = {
         "bound": "tensor" if t_tensor >= t_hbm else "hbm",
         "achieved": achieved_tflops, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
         "frac": achieved_tflops / peaks["bf16_tflops"],
-        # per launch of the fused kernel on this workload, from the committed `ncu` summary under profiles/
-        "traffic": fused_kernel_dram_traffic() if fused and not strong else None,
+        # per launch of the kernel that runs this workload, from the committed `ncu` summary under profiles/
+        "traffic": dram_traffic(_cabi.KERNEL_NAMES[kernel]) if not strong else None,
         "algorithmic_bytes": nbytes,
         "peak_source": peaks["source"] + " (burst cuBLAS bf16)",
-        "scope": "whole op = one launch per step; algorithmic FLOPs / ms_per_step; `stages` = the same "
-                 "stages launched one by one",
+        "scope": "whole op = one launch per step; algorithmic FLOPs / ms_per_step; `stages` = the same kernel's "
+                 "launch durations between events, with a host synchronisation after each call",
         "hbm_floor_frac": t_hbm / (ms_step * 1e-3),
         "stages": stages,
     }

@@ -225,8 +225,7 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
   // Status word and stage-completion counters start at zero.  The stage kernels that wait for nothing clear the
   // status word themselves: a memset in front of them is 1.5 us on the stream, as much as a small kernel.
   cudaError_t ce = cudaSuccess;
-  // (with per-stage times wanted, the tile kernels run one launch per stage)
-  const bool flow = L.kernel == MA_B200_KERNEL_TILE && stage_ms == nullptr && ma::flow_supported(g);
+  const bool flow = L.kernel == MA_B200_KERNEL_TILE && ma::flow_supported(g);
   if (flow || (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3 && L.kernel != MA_B200_KERNEL_HEAD_RESIDENT &&
                L.kernel != MA_B200_KERNEL_HEAD_FUSED && L.kernel != MA_B200_KERNEL_TILE)) {
     ce = cudaMemsetAsync(ws + L.status, 0, L.ar - L.status, stream);
@@ -272,24 +271,27 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
     return e;
   };
 
+  bool single = false;
+  auto one_launch = [&] {  // all stages in one launch: their time is the first entry, the others are 0
+    single = true;
+    if (ev != nullptr) cudaEventRecord(ev[1], stream);
+  };
+
   rc = MA_B200_OK;
   bool first = true;
   if (L.kernel == MA_B200_KERNEL_HEAD_FUSED || L.kernel == MA_B200_KERNEL_HEAD_RESIDENT) {
     ce = ma::launch_head_resident(g, p->qk_dtype, stream);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "head-resident kernel");
-    if (ev != nullptr)
-      for (int i = 1; i <= n_stages; ++i) cudaEventRecord(ev[i], stream);
+    one_launch();
   } else if (flow) {
     ce = ma::launch_flow(g, p->qk_dtype, counters, host_status, false, stream);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "tile kernels in one launch");
+    one_launch();
   } else if (L.kernel == MA_B200_KERNEL_TCGEN05) {
     // every stage in one persistent launch
     ce = ma::launch_fused(plan, g, counters, 0, n_stages, 1, 0, stream);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "fused kernel");
-    if (ev != nullptr) {
-      cudaEventRecord(ev[1], stream);
-      for (int i = 2; i <= n_stages; ++i) cudaEventRecord(ev[i], stream);
-    }
+    one_launch();
   } else {
   for (int t = 0; t + 1 < p->num_steps && rc == MA_B200_OK; ++t) {
     if ((ce = launch(ma::kStageRight, first)) != cudaSuccess) { rc = cuda_fail(ce, "right-factor stage"); break; }
@@ -305,8 +307,10 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
     if (rc == MA_B200_OK) {
       ce = cudaStreamSynchronize(stream);
       if (ce != cudaSuccess) rc = cuda_fail(ce, "cudaStreamSynchronize");
-      for (int i = 0; i < n_stages && i < n_stage_ms && rc == MA_B200_OK; ++i)
-        cudaEventElapsedTime(&stage_ms[i], ev[i], ev[i + 1]);
+      for (int i = 0; i < n_stages && i < n_stage_ms && rc == MA_B200_OK; ++i) {
+        stage_ms[i] = 0.f;
+        if (!single || i == 0) cudaEventElapsedTime(&stage_ms[i], ev[i], ev[i + 1]);
+      }
     }
     for (int i = 0; i <= n_stages; ++i) cudaEventDestroy(ev[i]);
     delete[] ev;
