@@ -54,3 +54,21 @@ def test_shards_return_the_bits_of_the_unsharded_call(E, H, N, D, B, T, hc, mask
     kernel = kernel_of_part(*part, mp, T, B, False, heads=E * H)
     got = ma.monarch_attention_b200(*part, mp, T, B, False, kernel=kernel)
     assert torch.equal(got.view(torch.int16), want[:1, :3].view(torch.int16))
+
+
+@pytest.mark.parametrize("N,B,H,T,name", [(4096, 64, 25, 2, "tcgen05-fused"), (4096, 64, 26, 2, "tile"), (16384, 128, 6, 3, "tcgen05-fused"),
+                                          (16384, 128, 7, 3, "tile"), (4096, 64, 9, 1, "tcgen05-fused"), (4096, 64, 12, 1, "tile")])
+def test_both_sides_of_the_line_between_fused_and_tile_kernels(N, B, H, T, name):
+    """5.5 tiles of 128 rows per SM and stage (148 SMs: 814), two with one iteration (296); either side matches the generic kernels."""
+    import monarch_attention_b200 as ma
+    from monarch_attention_b200 import _cabi
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the head counts are those around the line of 148 SMs")
+    dev = torch.device("cuda:0")
+    q, k, v, _ = _inputs(1, H, N, 64, False)
+    q, k, v = (t.to(dev) for t in (q, k, v))
+    assert _cabi.KERNEL_NAMES[_family(q, None, T, B)] == name
+    out = ma.MonarchAttention(B, T, "post")(q, k, v).float()
+    ref = ma.MonarchAttention(B, T, "post", impl="b200-generic")(q, k, v).float()
+    # (16-bit results of the same rounding points summed in different orders: the parity bound of the library)
+    assert ((out - ref).norm() / ref.norm()).item() <= 1e-2

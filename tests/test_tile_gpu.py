@@ -95,3 +95,24 @@ def test_expired_wait_ends_the_launch_and_is_reported(E, H, N, B, T):
         mod(q, k, v)
     assert lib.ma_b200_poll_device_status(0) == _cabi.OK
     assert torch.equal(mod(q, k, v), good)
+
+
+def test_full_size_tile_kernels():
+    """The headline size (16 heads of 16384 tokens): constant rows of V come back (the matrix is row-stochastic), heads may
+    change places without changing a bit, calls repeat, and two heads agree with the CPU oracle."""
+    import monarch_attention_b200 as ma
+    from oracle.monarch_oracle import monarch_attention_oracle
+    g = torch.Generator().manual_seed(1234)
+    dev = torch.device("cuda:0")
+    q, k, v = (torch.randn(1, 16, 16384, 64, generator=g).to(torch.bfloat16).to(dev) for _ in range(3))
+    mod = ma.MonarchAttention(128, 2, "post", impl="b200-tile")
+    c = torch.linspace(-2, 2, 64, device=dev).to(torch.bfloat16)
+    assert (mod(q, k, c.expand_as(v).contiguous()).float() - c.float()).abs().max().item() < 3e-2
+    out = mod(q, k, v)
+    for _ in range(3):
+        assert torch.equal(mod(q, k, v), out)
+    perm = torch.randperm(16, generator=g).to(dev)
+    assert torch.equal(mod(q[:, perm], k[:, perm], v[:, perm]), out[:, perm])
+    for h in (0, 11):
+        ref = monarch_attention_oracle(*(t[:, h:h + 1].cpu() for t in (q, k, v)), None, 2, 128, False).float()
+        assert ((out[:, h:h + 1].cpu().float() - ref).norm() / ref.norm()).item() <= 1e-2
