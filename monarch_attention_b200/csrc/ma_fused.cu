@@ -880,6 +880,10 @@ int* host_status_word(int device) {
   HostStatus& hs = g_host_status[device];
   if (!hs.tried) {
     hs.tried = true;
+    // The first call on a device may come while this thread captures a stream: an allocation would invalidate the capture
+    // unless the thread says that it does not belong to it.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
     void* hp = nullptr;
     if (cudaHostAlloc(&hp, 64, cudaHostAllocMapped) == cudaSuccess) {
       *reinterpret_cast<int*>(hp) = 0;
@@ -891,6 +895,7 @@ int* host_status_word(int device) {
         cudaFreeHost(hp);
       }
     }
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
     (void)cudaGetLastError();
   }
   return hs.dev;
