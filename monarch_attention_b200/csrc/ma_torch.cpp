@@ -173,6 +173,16 @@ struct AttentionFunction : torch::autograd::Function<AttentionFunction> {
   }
 };
 
+// int(x): block sizes and iteration counts of a configuration may be floats.
+int64_t as_integer(PyObject* x) {
+  if (PyLong_Check(x)) return PyLong_AsLongLong(x);
+  PyObject* i = PyNumber_Long(x);
+  if (i == nullptr) return -1;
+  const int64_t value = PyLong_AsLongLong(i);
+  Py_DECREF(i);
+  return value;
+}
+
 // forward(q, k, v, mask | None, T, B, pre_pad, kernel, out | None, token_major) -> Tensor, or None when an input
 // requires a gradient that the backward kernels do not give.
 PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -186,8 +196,9 @@ PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     mask_in = THPVariable_Unpack(args[3]);
   }
   Call c;
-  c.T = PyLong_AsLongLong(args[4]);
-  c.B = PyLong_AsLongLong(args[5]);
+  c.T = as_integer(args[4]);
+  c.B = as_integer(args[5]);
+  if (PyErr_Occurred()) return nullptr;
   c.pre_pad = PyObject_IsTrue(args[6]) == 1;
   c.kernel = (int)PyLong_AsLong(args[7]);
   Tensor out;

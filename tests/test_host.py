@@ -107,6 +107,19 @@ def test_module_api_mirrors_reference(lib):
         m(q[0], q[0], q[0])
 
 
+def test_block_size_and_steps_are_taken_as_integers(lib):
+    """Configurations hold floats and numpy integers too; the call gets as far as the check of the device."""
+    import numpy as np
+    from monarch_attention_b200 import MonarchAttention
+    q = torch.zeros(1, 2, 32, 16)
+    for B, T in ((16.0, 2.0), (np.int64(16), np.int32(2)), (torch.tensor(16), torch.tensor(2)), (np.float32(16), True)):
+        with pytest.raises(RuntimeError, match="no CPU path"):
+            MonarchAttention(B, T, "post")(q, q, q)
+    for B in (None, "x"):
+        with pytest.raises((TypeError, ValueError)):
+            MonarchAttention(B, 2, "post")(q, q, q)
+
+
 def test_unit_range_partitions():
     from monarch_attention_b200.sharding import unit_range
     for total in (0, 1, 7, 16, 768):
