@@ -1,5 +1,7 @@
-// tcgen05 stage kernels for 16-bit tensors with block size and block count from 33 to 256 and D <= 64: persistent CTAs,
-// three per SM (two for 256 keys), each on one 128-row tile at a time with one thread per tile row and a control warp.
+// tcgen05 stage kernels for 16-bit tensors and D <= 64, one launch per stage: persistent CTAs, three per SM (two for 256 keys),
+// each on one 128-row tile at a time with one thread per tile row and a control warp.  They take the calls whose block size
+// or block count is above 128 (the instances for 64 and 128 keys: the other side of such a call); up to 128 on both sides
+// all stages are one launch of ma_flow.inc.
 //
 // A tile is one key block m (or two, of up to 64 tokens) in the right-factor stages, one column j (or two) in the
 // left-factor and output stages.  A CTA loads its operands by TMA, forms S = A B^T in tensor memory, turns it row by row
@@ -12,9 +14,10 @@
 //                  them, and cr[m] is a sum along a thread's own row, before rounding, in fp32   (:26-35)
 // A thread owns a whole row, so no statistics are exchanged, and everything a warp does is a plain instruction stream;
 // the waits of one CTA (loads, tensor pipe, tensor memory) are covered by the other CTAs of the SM instead of by a
-// pipeline of specialised warps.  What bounds it: the exponentials, 16 per clock and SM, are 1024 cycles per 128 x 128
-// tile (2048 in the left-factor stage); measured, a tile takes about 7700 cycles from its S to its stores with three CTAs
-// sharing the SM (2600 per tile), most of it the latency of the chain S - P - O - store.  (Rows stored by their threads
+// pipeline of specialised warps.  What bounds it: at 256 keys the latency of the row passes, with eight row warps on an SM.  A
+// right-factor tile of 128 x 256 takes its CTA 11600 cycles (16 heads of 65536 tokens: 8192 tiles on 296 places in 163 us; the
+// stages of two iterations 163, 258, 196, 165), 5800 of the SM's per tile, of which the exponentials, 16 per clock and SM,
+// are 2048.  (Rows stored by their threads
 // instead of by TMA took 1700 cycles of that chain; launching the next stage early, by programmatic dependent launch,
 // cost the running stage its instruction cache: 18000 cycles for the first tile instead of 9000.)
 //

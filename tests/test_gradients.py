@@ -1,5 +1,6 @@
-"""Gradients: the library differentiates by recomputation (monarch_attention_b200/backward.py); the
-reference differentiates its eager implementation with autograd.  tests/golden holds the reference's own
+"""Gradients: the module's come from the backward kernels (csrc/ma_backward.cu), or from a recomputation in tensor operations
+where those do not apply (monarch_attention_b200/backward.py); the reference differentiates its eager implementation with
+autograd.  tests/golden holds the reference's own
 gradients on seeded cases (generated by tests/golden/make_golden.py)."""
 import numpy as np
 import pytest
