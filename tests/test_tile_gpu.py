@@ -65,7 +65,8 @@ def test_single_launch_stages_read_what_the_stage_before_wrote(H, B, M, T):
 
 
 @pytest.mark.parametrize("E,H,N,B,T", [(1, 2, 4096, 64, 2), (2, 12, 4096, 64, 1), (1, 3, 128 * 100 - 5, 128, 3),
-                                       (1, 2, 40 * 100, 40, 2), (1, 2, 200 * 40, 200, 2), (1, 1, 256 * 256, 256, 1)])
+                                       (1, 2, 40 * 100, 40, 2), (1, 2, 200 * 40, 200, 2), (1, 1, 256 * 256, 256, 1),
+                                       (1, 2, 40 * 200, 40, 2), (1, 2, 100 * 150, 100, 1)])
 def test_expired_wait_ends_the_launch_and_is_reported(E, H, N, B, T):
     """Single launch: the first stage is left out, so the waits for it run out; one launch per stage (blocks above 128): an
     operand is never asked for.  Every CTA gives up by itself, the status words say so, the next call raises, and the one
