@@ -17,6 +17,14 @@ constexpr float kLn2 = 0.6931471805599453f;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// One lane of the warp, always the same one.  (Behind it the compiler knows that a tensor instruction is issued once for the
+// warp and keeps its operands in uniform registers; behind a test of the lane's number it moves them there one by one, some
+// 150 cycles for each instruction of a starved warp.)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r)::"memory");
+  return r != 0;
+}
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }

@@ -203,21 +203,25 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(NK))
     // S = A B^T over the features, both K-major
     auto issue_abt = [&](uint32_t a, uint32_t b) {
       tc_fence_after();
-      if (lane == 0) {
-        constexpr uint32_t idesc = instr_desc(kFmt, 0, 0, kCols, kRows);
-        const uint32_t da = smem_desc_lo(a, 16), db = smem_desc_lo(b, 16);
-        for (int kk = 0; kk < (D + 15) / 16; ++kk) mma_f16_lo(tmem, da + kk * 2, db + kk * 2, idesc, kk > 0);
+      constexpr uint32_t idesc = instr_desc(kFmt, 0, 0, kCols, kRows);
+      const uint32_t da = smem_desc_lo(a, 16), db = smem_desc_lo(b, 16);
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          if (16 * kk < D) mma_f16_lo(tmem, da + kk * 2, db + kk * 2, idesc, kk > 0);
         mma_commit(bar(kBarS));
       }
     };
     // O[128 x 64] = P X, P in tensor memory, X row-major [keys][64]
     auto issue_px = [&](uint32_t x) {
       tc_fence_after();
-      if (lane == 0) {
-        constexpr uint32_t idesc = instr_desc(kFmt, 0, 1, 64, kRows);
-        const uint32_t dx = smem_desc_lo(x, kRows * kRowBytes);
-        const int steps = kUnits == 2 ? 8 : (keys + 15) >> 4;
-        for (int kk = 0; kk < steps; ++kk) mma_f16_ts(tmem + kTmemO, tmem + kk * 8, dx + kk * 128, idesc, kk > 0);
+      constexpr uint32_t idesc = instr_desc(kFmt, 0, 1, 64, kRows);
+      const uint32_t dx = smem_desc_lo(x, kRows * kRowBytes);
+      const int steps = kUnits == 2 ? 8 : (keys + 15) >> 4;
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < kCols / 16; ++kk)
+          if (kk < steps) mma_f16_ts(tmem + kTmemO, tmem + kk * 8, dx + kk * 128, idesc, kk > 0);
         mma_commit(bar(kBarO));
       }
     };
@@ -314,7 +318,9 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(NK))
         for (int i = max(la - na, HOLD ? 1 : 0); i < la; ++i) (void)mbar_wait(bar(kBarA + (kTwoA ? i & 1 : 0)), (uint32_t)(kTwoA ? i >> 1 : i) & 1u);
         for (int i = max(lb - nb, 0); i < lb; ++i) (void)mbar_wait(bar(kBarB + (kTwoB ? i & 1 : 0)), (uint32_t)(kTwoB ? i >> 1 : i) & 1u);
         if (lv > 0) (void)mbar_wait(bar(kBarV), (uint32_t)(lv - 1) & 1u);
-        // the contractions that were issued have read their operands and written tensor memory
+      }
+      __syncwarp();
+      if (elect_one()) {  // the contractions that were issued have read their operands and written tensor memory
         mma_commit(bar(kBarDrain));
         (void)mbar_wait(bar(kBarDrain), 0);
       }
