@@ -458,10 +458,13 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(NK))
       const bool masked = plain ? false : named_barrier_or(kRowBarrier, kRows, missing);
       column_vector(i + 1, next_vec);
       row_scalar(i + 1, next_row);
-      // Shift of a column row: the maximum of S, plus a bound on -cl (an entropy of at most 256 outcomes: 8 in powers of
-      // two).  Any shift within a few powers of two of the true maximum gives the same quotients.
-      auto column_shift = [&] {
-        return masked ? row_max<true>(t_s, nch, my_vec, kLog2e) : fmaf(row_max<false>(t_s, nch, my_vec, 1.0f), kLog2e, 8.0f);
+      // e over S (STORE) and its sum, against a shift: the maximum of S, plus a bound on -cl (an entropy of at most 256 outcomes: 8 in
+      // powers of two).  Any shift within a few powers of two of the true maximum gives the same quotients.
+      auto column_sum = [&](auto store, float& off) {
+        constexpr bool kStore = decltype(store)::value;
+        if (masked) return masked_column_exps<T, kStore>(t_s, nch, my_vec, off);
+        off = fmaf(row_max<false>(t_s, nch, my_vec, 1.0f), kLog2e, 8.0f);
+        return column_exps<T, kStore>(t_s, nch, my_vec, off);
       };
 
       ok = wait(kBarS, ns++);
@@ -490,8 +493,8 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(NK))
 
       if (KIND == kStageOutput) {
         if (warp_live) {
-          const float off = column_shift();
-          normalise<T>(t_s, t_p, nch, rcp_fast(column_exps<T, true>(t_s, nch, my_vec, off)));
+          float off;
+          normalise<T>(t_s, t_p, nch, rcp_fast(column_sum(std::true_type(), off)));
           zero_rest();
         }
         p_ready();
@@ -512,8 +515,8 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(NK))
           }
           float z = 1e30f;  // 2^-z = 0: rows that do not exist and invalid queries contribute nothing
           if (warp_live) {
-            const float off = column_shift();
-            const float sum = column_exps<T, false>(t_s, nch, my_vec, off);
+            float off;
+            const float sum = column_sum(std::false_type(), off);
             if (my_row[rc] != 0.f) z = off + lg2(sum);
           }
           lse[tid + rc * kRows] = z;
