@@ -23,4 +23,5 @@
 // Explicit launcher templates are declared before use in ma_warp_kernels.inc and defined in
 // ma_warp_wide.inc, so the public entry points have to come last.
 #include "ma_warp_kernels.inc"
+#include "ma_warp_head.inc"
 #include "ma_warp_wide.inc"

@@ -92,37 +92,58 @@ __device__ __forceinline__ int reduce_rows(float (&v)[N], int lane) {
   return base;
 }
 
-// Copies `rows` rows of `width` elements (a multiple of 8) into a shared tile with row
-// pitch `pitch` elements, zero-filling rows that do not exist, columns past width and rows
-// [rows, rpad).  Threads tid of nthreads cooperate.  The copies are asynchronous (cp.async, 16 bytes
-// each, zero-fill by giving a source size of 0): a thread queues all of its pieces without waiting;
-// tiles_commit_and_wait() must be called before the tile is read.
+// Copies `rows` rows of `width` elements (whole 16-byte pieces) into a shared tile with row pitch `pitch` elements,
+// zero-filling rows that do not exist, columns past width and rows [rows, rpad).  Threads tid of nthreads cooperate.  The
+// copies are asynchronous (cp.async, 16 bytes each, zero-fill by giving a source size of 0): a thread queues all of its
+// pieces without waiting; tiles_commit_and_wait() must be called before the tile is read.
 // Every source these kernels have is an arithmetic progression of rows: row r comes from element
 // offset (n0 + r*nstep)*row_stride of `base` and exists iff r < rows and 0 <= n0 + r*nstep < n_limit
 // (token index inside the sequence; for the dense state tensors n0 = 0, nstep = 1, n_limit = rows).
-// Row, column chunk, token index and source offset are carried from one 16-byte piece to the next
-// with additions only.
+// fp32: eight threads share a row, and a thread takes every eighth piece of it, so that all but the first of a row's copies
+// differ from it by constants.  The fp32 stage kernels are bound by their instructions, and those that worked out a row and a
+// column for every piece were 300 of 2530 (16 x 16 x 72) for each tile (67.3 instead of 72 us for 128 heads of 256 x 72, three
+// iterations).  16-bit types, whose rows are one or two lines: one piece after the other, with row, column chunk, token index
+// and source offset carried along by additions only; shared rows were slower there (64 x 12 heads of 197 x 64: 39.1 instead of
+// 37.1 us; 8 x 16 of 2025 x 80: 115 instead of 107).
 template <typename T, int CHUNKS>  // CHUNKS: 16-byte pieces of a padded row
 __device__ __forceinline__ void load_rows(T* tile, int pitch, int rows, int rpad, int width, const T* base, int n0,
                                           int nstep, int n_limit, long long row_stride, int tid, int nthreads,
                                           const void* any_valid_global) {
   constexpr int kPer = 16 / (int)sizeof(T);  // elements of a piece
-  int r = tid / CHUNKS, c = tid - r * CHUNKS;
-  const int dr = nthreads / CHUNKS, dc = nthreads - dr * CHUNKS;
-  int n = n0 + r * nstep;
-  const T* src = base + (long long)n * row_stride;
-  uint32_t dst = smem_addr(tile + r * pitch);
-  const int dn = dr * nstep;
-  const long long dsrc = (long long)dn * row_stride, step1 = (long long)nstep * row_stride;
-  const uint32_t ddst = (uint32_t)(dr * pitch) * (uint32_t)sizeof(T), dst1 = (uint32_t)pitch * (uint32_t)sizeof(T);
-  while (r < rpad) {
-    const bool ok = r < rows && c * kPer < width && (unsigned)n < (unsigned)n_limit;
-    const void* gsrc = ok ? static_cast<const void*>(src + c * kPer) : any_valid_global;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(c << 4)), "l"(gsrc),
-                 "r"(ok ? 16u : 0u)
-                 : "memory");
-    c += dc; r += dr; n += dn; src += dsrc; dst += ddst;
-    if (c >= CHUNKS) { c -= CHUNKS; ++r; n += nstep; src += step1; dst += dst1; }
+  if constexpr (sizeof(T) == 4) {
+    constexpr int L = 8;
+    const int q = tid % L;
+    for (int r = tid / L; r < rpad; r += nthreads / L) {
+      const int n = n0 + r * nstep;
+      const bool ok = r < rows && (unsigned)n < (unsigned)n_limit;
+      const T* src = (ok ? base + (long long)n * row_stride : static_cast<const T*>(any_valid_global)) + q * kPer;
+      const uint32_t dst = smem_addr(tile + r * pitch + q * kPer);
+#pragma unroll
+      for (int c = 0; c < CHUNKS; c += L) {
+        if (c + L > CHUNKS && c + q >= CHUNKS) break;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 16u * c), "l"(src + c * kPer),
+                     "r"(ok && (c + q) * kPer < width ? 16u : 0u)
+                     : "memory");
+      }
+    }
+  } else {
+    int r = tid / CHUNKS, c = tid - r * CHUNKS;
+    const int dr = nthreads / CHUNKS, dc = nthreads - dr * CHUNKS;
+    int n = n0 + r * nstep;
+    const T* src = base + (long long)n * row_stride;
+    uint32_t dst = smem_addr(tile + r * pitch);
+    const int dn = dr * nstep;
+    const long long dsrc = (long long)dn * row_stride, step1 = (long long)nstep * row_stride;
+    const uint32_t ddst = (uint32_t)(dr * pitch) * (uint32_t)sizeof(T), dst1 = (uint32_t)pitch * (uint32_t)sizeof(T);
+    while (r < rpad) {
+      const bool ok = r < rows && c * kPer < width && (unsigned)n < (unsigned)n_limit;
+      const void* gsrc = ok ? static_cast<const void*>(src + c * kPer) : any_valid_global;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(c << 4)), "l"(gsrc),
+                   "r"(ok ? 16u : 0u)
+                   : "memory");
+      c += dc; r += dr; n += dn; src += dsrc; dst += ddst;
+      if (c >= CHUNKS) { c -= CHUNKS; ++r; n += nstep; src += step1; dst += dst1; }
+    }
   }
 }
 __device__ __forceinline__ void tiles_commit_and_wait() {
@@ -373,14 +394,27 @@ __device__ __forceinline__ void warp_gemm_pv(float (&o)[DP / 8][4], const Factor
   }
 }
 
-// Writes a warp's 16 x D accumulator tile to global rows: fragments go to a 16-row staging area in
-// shared memory (the warp's own, no longer needed operand rows), then every lane copies 16-byte
-// pieces, so that each 128-byte row is written by eight consecutive lanes.  row_ptr(r) gives the
-// destination of row r (0..15) or nullptr to skip it.
+// Writes a warp's 16 x D accumulator tile to global rows; row_ptr(r) gives the destination of row r (0..15) or nullptr to
+// skip it.  fp32: straight from the fragments, four lanes writing 32 consecutive bytes of a row.  16-bit types: the fragments
+// go to a 16-row staging area in shared memory (the warp's own, no longer needed operand rows), then every lane copies 16-byte
+// pieces, so that each 128-byte row is written by eight consecutive lanes.
 template <typename T, int DP, int PITCH, typename RowFn>
 __device__ __forceinline__ void store_rows(const float (&o)[DP / 8][4], T* stage, RowFn row_ptr, int D, int lane,
                                            float post_scale, bool double_round) {
   const int gq = lane >> 2, t = lane & 3;
+  if constexpr (sizeof(T) == 4) {
+    T* const rows[2] = {row_ptr(gq), row_ptr(gq + 8)};
+    __syncwarp();
+#pragma unroll
+    for (int nt = 0; nt < DP / 8; ++nt) {
+      const int c = nt * 8 + 2 * t;
+      if (c >= D) break;
+      if (rows[0] != nullptr) Tile<T>::store_pair(rows[0] + c, o[nt][0] * post_scale, o[nt][1] * post_scale);
+      if (rows[1] != nullptr) Tile<T>::store_pair(rows[1] + c, o[nt][2] * post_scale, o[nt][3] * post_scale);
+    }
+    __syncwarp();
+    return;
+  }
   // The reference rounds the product to storage before scaling it (ma/ma_torch.py:21).  Scaling by a power
   // of two (1/sqrt(D) for D = 16, 64, 256) commutes with rounding, so one rounding gives the same bits.
   const bool two_roundings = double_round && (__float_as_uint(post_scale) & 0x007fffffu) != 0u;
