@@ -223,11 +223,12 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
     return fail(MA_B200_CUDA_ERROR, std::string(what) + ": " + cudaGetErrorString(e));
   };
   // Status word and stage-completion counters start at zero.  The stage kernels that wait for nothing clear the
-  // status word themselves: a memset in front of them is 1.5 us on the stream, as much as a small kernel.
+  // status word themselves (a memset in front of them is 1.5 us on the stream, as much as a small kernel), and the
+  // single-launch tile kernels have a kernel before them that clears both.
   cudaError_t ce = cudaSuccess;
   const bool flow = L.kernel == MA_B200_KERNEL_TILE && ma::flow_supported(g);
-  if (flow || (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3 && L.kernel != MA_B200_KERNEL_HEAD_RESIDENT &&
-               L.kernel != MA_B200_KERNEL_HEAD_FUSED && L.kernel != MA_B200_KERNEL_TILE)) {
+  if (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3 && L.kernel != MA_B200_KERNEL_HEAD_RESIDENT &&
+      L.kernel != MA_B200_KERNEL_HEAD_FUSED && L.kernel != MA_B200_KERNEL_TILE) {
     ce = cudaMemsetAsync(ws + L.status, 0, L.ar - L.status, stream);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(status, counters)");
   }
