@@ -587,7 +587,8 @@ def run_ours(args, rank, world, local):
                 "api": "monarch_attention_b200_host(streamed=True): pinned host q, k, v in, pinned host result out every "
                        f"step, {args.e2e_heads_per_chunk} heads per chunk; the copy-in of a step overlaps the kernels and "
                        "the copy-out of the step before it"},
-        "gpu_launches": args.steps * (1 if one_launch else n_stage),
+        # (the single-launch tile kernel has a kernel before it that clears its counters)
+        "gpu_launches": args.steps * (2 if kernel == _cabi.KERNEL_TILE else 1 if one_launch else n_stage),
         "roofline": roofline,
         "cpu_baseline": cpu_baseline,
         "context": context,

@@ -113,7 +113,7 @@ typedef struct ma_b200_problem {
  * ar: (E*H, M, B, D) qk_dtype   cr: (E*H, M, B) f32
  * al: (E*H, B, M, D) qk_dtype   cl: (E*H, B, M) f32   y: (E*H, B, M, Dv) v_dtype
  * status: one int32 device flag, 0 = no device-side error.
- * counters: (E*H, 2T) int32 stage-completion counters of the fused kernel. */
+ * counters: (E*H, 2T) int32 stage-completion counters of the fused and the single-launch tile kernel. */
 typedef struct ma_b200_workspace_layout {
   size_t status, counters, ar, cr, al, cl, y, total;
   int32_t M;
@@ -158,7 +158,8 @@ MA_B200_API int ma_b200_forward_typed_mask(const ma_b200_problem* p, int mask_ty
  * and, after synchronising the stream, writes the stage durations in milliseconds to
  * stage_ms[0 .. min(n_stage_ms, 2*num_steps) - 1] in launch order (a family that takes
  * all stages in one launch - the fused, head-resident and, up to blocks of 128, the tile kernels - has its duration in
- * stage_ms[0], the other entries are 0).  The kernels timed are the ones ma_b200_forward launches.  Blocks the host.
+ * stage_ms[0], the other entries are 0; the fp32 tensor path's single launch is run once for each stage here).  The kernels
+ * timed are the ones ma_b200_forward launches.  Blocks the host.
  * reference: the per-kernel NVTX/ncu harness, perfbench/bench.py:199-223. */
 MA_B200_API int ma_b200_forward_timed(const ma_b200_problem* p, void* workspace, size_t workspace_bytes, void* stream,
                           float* stage_ms, int32_t n_stage_ms);
