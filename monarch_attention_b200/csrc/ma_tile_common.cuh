@@ -181,6 +181,7 @@ __device__ __forceinline__ float column_exps(uint32_t t_s, int nch, const float*
 }
 
 constexpr float kFar = 1048576.f;
+constexpr float kLeastShift = 0.1f * kGone;
 
 template <int N>
 __device__ __forceinline__ float max_of(const float (&v)[N]) {
@@ -188,9 +189,7 @@ __device__ __forceinline__ float max_of(const float (&v)[N]) {
   m.take(v);
   return m.get();
 }
-__device__ __forceinline__ bool any_far(const Sum2& s) {
-  return __any_sync(0xffffffffu, fmaxf(fmaxf(s.a.x, s.a.y), fmaxf(s.b.x, s.b.y)) > kFar);
-}
+__device__ __forceinline__ bool is_far(const Sum2& s) { return fmaxf(fmaxf(s.a.x, s.a.y), fmaxf(s.b.x, s.b.y)) > kFar; }
 // The columns before piece c times f.
 __device__ __forceinline__ void scale_columns(uint32_t t_s, int c, float f) {
   tmem_wait_st();
@@ -211,7 +210,8 @@ __device__ __forceinline__ void scale_columns(uint32_t t_s, int c, float f) {
 // quotients, so it is taken from the first 16 columns, and raised to the maximum of later ones (what was formed before is scaled
 // down) where a sum of 16 passes 2^20; a row sum in fp32 is good to 2^127, so nothing has been lost by then.  48 heads of 7683
 // tokens, blocks of 64: 145 us instead of 154.  (Where no column is missing the pass of its own is as fast: the check costs
-// what it saves.)  STORE: e over S.
+// what it saves.)  Logits below the range of the storage type are -inf, and 16 such columns would make the shift -inf and e NaN:
+// it stays above kLeastShift, far below any other logit and far above a missing column's.  STORE: e over S.
 template <typename T, bool STORE>
 __device__ __forceinline__ float masked_column_exps(uint32_t t_s, int nch, const float* bias, float& off) {
   Sum2 s;
@@ -241,13 +241,14 @@ __device__ __forceinline__ float masked_column_exps(uint32_t t_s, int nch, const
       }
     };
     logits();
-    if (c == 0) off = max_of(v);
+    if (c == 0) off = fmaxf(max_of(v), kLeastShift);
     exps();
-    if (any_far(cs)) {
+    const bool far = is_far(cs);
+    if (__any_sync(0xffffffffu, far)) {
       tmem_ld16_nowait(t_s + 16 * c, v);
       tmem_wait_ld16(v);
       logits();
-      const float to = fmaxf(max_of(v), off), f = ex2(off - to);
+      const float to = far ? fmaxf(max_of(v), off) : off, f = ex2(off - to);  // (a row goes by its own columns: f = 1 in the others)
       if (STORE) scale_columns(t_s, c, f);
       s.a = mul2(s.a, make_float2(f, f));
       s.b = mul2(s.b, make_float2(f, f));
