@@ -157,9 +157,9 @@ MA_B200_API int ma_b200_forward_typed_mask(const ma_b200_problem* p, int mask_ty
 /* Same as ma_b200_forward, and additionally records one CUDA event pair per stage launch
  * and, after synchronising the stream, writes the stage durations in milliseconds to
  * stage_ms[0 .. min(n_stage_ms, 2*num_steps) - 1] in launch order (a family that takes
- * all stages in one launch - the fused, head-resident and, up to blocks of 128, the tile kernels - has its duration in
- * stage_ms[0], the other entries are 0; the fp32 tensor path's single launch is run once for each stage here).  The kernels
- * timed are the ones ma_b200_forward launches.  Blocks the host.
+ * all stages in one launch - the fused, head-resident and, up to blocks of 128, the tile kernels, and the fp32 tensor path
+ * for few heads with blocks up to 32 - has its duration in stage_ms[0], the other entries are 0).  The kernels timed are the
+ * ones ma_b200_forward launches.  Blocks the host.
  * reference: the per-kernel NVTX/ncu harness, perfbench/bench.py:199-223. */
 MA_B200_API int ma_b200_forward_timed(const ma_b200_problem* p, void* workspace, size_t workspace_bytes, void* stream,
                           float* stage_ms, int32_t n_stage_ms);

@@ -258,15 +258,12 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
     cudaEventRecord(ev[0], stream);
   }
   int stage_idx = 0;
-  // (a timed call runs the single launch of the fp32 tensor path stage by stage)
-  const bool head_f32 = L.kernel == MA_B200_KERNEL_TF32X3 && ma::head_f32_pays(g);
   auto launch = [&](ma::StageKind kind, bool first) -> cudaError_t {
     cudaError_t e;
     if (L.kernel == MA_B200_KERNEL_TCGEN05_STAGED)
       e = ma::launch_fused(plan, g, counters, stage_idx, stage_idx + 1, 0, 0, stream);
     else if (L.kernel == MA_B200_KERNEL_TILE)
       e = ma::launch_tile_stage(g, p->qk_dtype, kind, first, host_status, false, stream);
-    else if (head_f32) e = ma::launch_head_f32(g, stage_idx, stage_idx + 1, stream);
     else if (L.kernel == MA_B200_KERNEL_WARP_MMA || L.kernel == MA_B200_KERNEL_TF32X3)
       e = ma::launch_warp_stage(g, p->qk_dtype, kind, first, stream);
     else e = ma::launch_generic_stage(g, p->qk_dtype, p->v_dtype, kind, first, stream);
@@ -287,9 +284,10 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
     ce = ma::launch_head_resident(g, p->qk_dtype, stream);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "head-resident kernel");
     one_launch();
-  } else if (head_f32 && ev == nullptr) {
-    ce = ma::launch_head_f32(g, 0, n_stages, stream);
+  } else if (L.kernel == MA_B200_KERNEL_TF32X3 && ma::head_f32_pays(g)) {
+    ce = ma::launch_head_f32(g, stream);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "fp32 tensor path in one launch");
+    one_launch();
   } else if (flow) {
     ce = ma::launch_flow(g, p->qk_dtype, counters, host_status, false, stream);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "tile kernels in one launch");

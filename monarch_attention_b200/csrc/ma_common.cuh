@@ -176,9 +176,9 @@ struct TcPlan;
 int tc_plan_get(const Geometry& g, int qk_dtype, TcPlan* plan, const char** err);
 int tc_plan_create(const Geometry& g, int qk_dtype, TcPlan** plan, const char** err);
 void tc_plan_destroy(TcPlan* plan);
-// Stages [stage0, stage1) of the fp32 tensor path (TF32X3) in one launch, for block size and count up to 32 (ma_warp_head.inc).
+// All stages of the fp32 tensor path (TF32X3) in one launch, for block size and count up to 32 (ma_warp_head.inc).
 bool head_f32_pays(const Geometry& g);
-cudaError_t launch_head_f32(const Geometry& g, int stage0, int stage1, cudaStream_t stream);
+cudaError_t launch_head_f32(const Geometry& g, cudaStream_t stream);
 // Persistent fused kernel: stages [stage_begin, stage_end) of the 2T stages in one cooperative launch.
 size_t fused_counter_bytes(const Geometry& g);
 // (spin_limit: iterations of the dependency wait before it gives up, 0 = default; for the wait-expiry self-test.)

@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
     (1, 2, 200 * 40, 64, 200, 2, torch.bfloat16, 4),    # tile kernels, a launch per stage
     (1, 2, 4096, 64, 64, 2, torch.bfloat16, 1),         # fused kernel
     (8, 12, 197, 64, 15, 2, torch.bfloat16, 1),         # head-resident kernel
-    (2, 3, 250, 64, 16, 2, torch.float32, 4)])          # fp32 stage kernels
+    (2, 3, 250, 64, 16, 2, torch.float32, 1),           # fp32 tensor path, one launch
+    (50, 6, 250, 64, 16, 2, torch.float32, 4)])         # ... a launch per stage
 def test_timed_forward_runs_the_kernels_of_the_forward(E, H, N, D, B, T, dtype, launches):
     from monarch_attention_b200 import _cabi
     from monarch_attention_b200.monarch_attention import make_problem
