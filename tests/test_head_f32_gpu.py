@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("few,many,N,D,B,T,pad,masked", [
     (1, 150, 256, 72, 16, 3, "post", False), (100, 150, 15 * 14 - 3, 64, 15, 2, "pre", True), (3, 2100, 1, 24, 1, 1, "post", False),
     (2, 300, 9 * 16 - 8, 80, 9, 2, "post", False), (129, 160, 16 * 16, 32, 16, 1, "pre", True),
-    (1, 16, 1024, 64, 32, 2, "post", False), (3, 30, 17 * 30 - 9, 72, 17, 3, "pre", True), (5, 40, 32 * 10 - 1, 40, 32, 2, "post", True)])
+    (1, 16, 1024, 64, 32, 2, "post", False), (3, 30, 17 * 30 - 9, 72, 17, 3, "pre", True), (5, 40, 32 * 10 - 1, 40, 32, 2, "post", True),
+    (140, 150, 256, 64, 16, 3, "post", False), (30, 40, 24 * 23 - 5, 64, 24, 2, "pre", True)])
 def test_single_launch_returns_the_bits_of_the_stage_kernels(few, many, N, D, B, T, pad, masked):
     import monarch_attention_b200 as ma
     from oracle.monarch_oracle import monarch_attention_oracle

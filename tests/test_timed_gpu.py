@@ -15,7 +15,11 @@ pytestmark = pytest.mark.gpu
     (1, 2, 4096, 64, 64, 2, torch.bfloat16, 1),         # fused kernel
     (8, 12, 197, 64, 15, 2, torch.bfloat16, 1),         # head-resident kernel
     (2, 3, 250, 64, 16, 2, torch.float32, 1),           # fp32 tensor path, one launch
-    (50, 6, 250, 64, 16, 2, torch.float32, 4)])         # ... a launch per stage
+    (50, 6, 250, 64, 16, 2, torch.float32, 4),          # ... a launch per stage
+    # ... while the GPU holds the clusters of all heads at once, whatever their blocks
+    (17, 8, 250, 64, 16, 2, torch.float32, 1), (20, 8, 100, 64, 10, 2, torch.float32, 4), (40, 8, 36, 64, 6, 1, torch.float32, 2),
+    # ... and blocks above 24 while each cluster has its SMs to itself
+    (1, 14, 1024, 64, 32, 2, torch.float32, 1), (2, 8, 625, 64, 25, 2, torch.float32, 4), (2, 13, 576, 64, 24, 2, torch.float32, 1)])
 def test_timed_forward_runs_the_kernels_of_the_forward(E, H, N, D, B, T, dtype, launches):
     from monarch_attention_b200 import _cabi
     from monarch_attention_b200.monarch_attention import make_problem
