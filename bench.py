@@ -517,7 +517,8 @@ def run_ours(args, rank, world, local):
     if strong:
         flops, nbytes = flops / world, nbytes / world  # this rank's share; the roofline below is per GPU
     names = ["right", "left", "right_with_v", "output"]
-    if kernel == _cabi.KERNEL_TILE:
+    one_launch = kernel == _cabi.KERNEL_TCGEN05 or not any(acc[1:])
+    if not any(acc[1:]):
         names, stage_flops = ["all_in_one_launch"], {"all_in_one_launch": sum(stage_flops.values())}
     stages = [{"stage": n, "ms": acc[i], "tflops": stage_flops[n] / (world if strong else 1) / (acc[i] * 1e-3) / 1e12}
               for i, n in enumerate(names)]
@@ -525,7 +526,8 @@ def run_ours(args, rank, world, local):
     t_tensor = flops / (peaks["bf16_tflops"] * 1e12)
     t_hbm = nbytes / (peaks["hbm_gbs"] * 1e9)
     achieved_tflops = flops / (ms_step * 1e-3) / 1e12
-    one_launch = kernel in (_cabi.KERNEL_TCGEN05, _cabi.KERNEL_TILE)
+    # kernels of a step: one a stage, or one for all of them, before which the tile kernels have one that clears their counters
+    launches = n_stage if not one_launch else 2 if kernel == _cabi.KERNEL_TILE else 1
     roofline = {
         "bound": "tensor" if t_tensor >= t_hbm else "hbm",
         "achieved": achieved_tflops, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
@@ -534,7 +536,7 @@ def run_ours(args, rank, world, local):
         "traffic": dram_traffic(_cabi.KERNEL_NAMES[kernel]) if not strong else None,
         "algorithmic_bytes": nbytes,
         "peak_source": peaks["source"] + " (burst cuBLAS bf16)",
-        "scope": "whole op = one launch per step; algorithmic FLOPs / ms_per_step; `stages` = the same kernel's "
+        "scope": f"whole op, {launches} kernel launch(es) per step; algorithmic FLOPs / ms_per_step; `stages` = the same kernel's "
                  "launch durations between events, with a host synchronisation after each call",
         "hbm_floor_frac": t_hbm / (ms_step * 1e-3),
         "stages": stages,
@@ -587,8 +589,7 @@ def run_ours(args, rank, world, local):
                 "api": "monarch_attention_b200_host(streamed=True): pinned host q, k, v in, pinned host result out every "
                        f"step, {args.e2e_heads_per_chunk} heads per chunk; the copy-in of a step overlaps the kernels and "
                        "the copy-out of the step before it"},
-        # (the single-launch tile kernel has a kernel before it that clears its counters)
-        "gpu_launches": args.steps * (2 if kernel == _cabi.KERNEL_TILE else 1 if one_launch else n_stage),
+        "gpu_launches": args.steps * launches,
         "roofline": roofline,
         "cpu_baseline": cpu_baseline,
         "context": context,
