@@ -34,7 +34,9 @@ print("family ok")
     ((1, 4, 4096, 64, 64, 2), "bfloat16"),      # fused kernel
     ((2, 12, 197, 64, 15, 2), "bfloat16"),      # head-resident kernel
     ((1, 2, 40 * 60, 80, 40, 2), "bfloat16"),   # warp-level kernels
-    ((2, 12, 256, 64, 16, 2), "float32"),       # fp32 stage kernels
+    ((2, 12, 256, 64, 16, 2), "float32"),       # fp32 tensor path, one launch
+    ((2, 13, 576, 64, 24, 2), "float32"),       # ... where a query decides whether the heads fit
+    ((20, 8, 256, 64, 16, 2), "float32"),       # ... a launch per stage
     ((1, 2, 250, 20, 16, 2), "float32")])       # generic kernels
 def test_first_call_of_a_process_can_be_captured(shape, dtype):
     run = subprocess.run([sys.executable, "-c", SCRIPT.format(root=ROOT, shape=shape, dtype=dtype)], capture_output=True, text=True,
