@@ -90,7 +90,10 @@ ma::Geometry make_geometry(const ma_b200_problem* p, int mask_type = MA_B200_MAS
 // narrow heads and few heads are better off with 16-row warps and two launches.  Microseconds of one iteration, from a
 // sweep of blocks and counts of 16 to 200, 4 to 256 heads and widths 32 and 64: a tile takes 12.5 ns of the GPU's time and an
 // iteration 18.6 us at the least (8 beside the tiles' own time); a padded element of a warp-level tile takes 2.4 ps (1.7 in
-// heads of up to 32), two launches 6 us.
+// heads of up to 32), two launches 6 us.  Measured again with the single-launch tile kernels' split roles, both families on blocks and
+// counts of 8 to 128, 4 to 256 heads, one and two iterations (675 calls): what the rule takes sums up to 0.5 % more than the
+// faster one of each call, and 23 calls lose more than 5 %: 128 x 16 x 64 the most, us, warp-level / tile with one iteration 52 / 43 at
+// 48 heads, 125 / 93 at 128, 239 / 173 at 256; 96 x 33 x 32 the other way, 22.8 / 26.9 at 16.
 bool warp_beats_tiles(const ma::Geometry& g, double heads) {
   if (g.B > 128 || g.M > 128) return false;  // (the warp-level kernels then walk a row twice: never the faster ones)
   auto up16 = [](int x) { return (x + 15) & ~15; };
@@ -135,10 +138,12 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, long long he
   const bool tf32_pays = tf32_ok && g.D >= 24;
   // The fused kernel takes one tile at a time through an SM, quickly; the tile kernels take four, each more slowly, and do
   // 1.2 to 1.4 times as many in a time.  So the fused kernel is the faster one while a stage is few rounds of one tile per
-  // SM.  Measured (us, fused / tile kernels) over 32 to 2048 tiles per stage, blocks of 64 and 128: with two iterations 42 / 45 at
-  // 3.5 tiles per SM, 50 / 54 and 59 / 63 at 5.2, 54.8 / 55.8 at 5.8, 56.9 / 56.2 at 6.1, 77 / 59 and 75 / 68 at 6.9; with three
-  // 70 / 73 and 83 / 91 at 5.2, 75.2 / 74.1 at 5.8, 79 / 75 at 6.1: the line is at 5.5.  With one, whose two stages leave the tile
-  // kernels' list fewer waits, 20.7 / 20.7 and 21.5 / 22.8 at 1.7, 23.1 / 22.8 and 26.6 / 25.0 at 2.6: at 2.
+  // SM.  Measured (us, fused / tile kernels, calls back to back on three sets of inputs) over 128 to 1536 tiles per stage, blocks
+  // of 64 and 128: with two iterations 42.0 / 44.0 and 47.1 / 51.6 at 3.5 tiles per SM, 49.7 / 50.6 and 59.2 / 62.3 at 5.2, 53.4 /
+  // 51.8 (blocks of 64) at 5.6, 57.3 / 52.9 and 68.2 / 65.0 at 6.1, 77 / 55 and 76 / 69 at 6.9; with three 69.8 / 69.6 and 82 / 90 at
+  // 5.2, 73.9 / 70.1 (64) at 5.6, 79 / 72 and 95 / 94 at 6.1: the line is at 5.5.  With one, whose two stages leave the tile kernels'
+  // list fewer waits, 16.5 / 18.5 and 18.5 / 18.7 at 0.9, 20.4 / 19.3 and 21.3 / 20.8 at 1.7, 22.7 / 21.8 and 24.9 / 24.7 at 2.6: the
+  // line at 2 was drawn before the roles of the tile kernels were split, and takes up to 5 % too long between 1 and 2.
   const bool few_tiles = tc_ok && heads * p->N / 64 <= (long long)ma::sm_count() * (p->num_steps == 1 ? 4 : 11);
   // Head widths other than 64 and 72 have one tile size for both kinds of stage in the head-resident kernel: with one side of
   // up to 16 beside a longer one the warp-level kernels pad less, and win once the heads no longer fit the SMs in one round.

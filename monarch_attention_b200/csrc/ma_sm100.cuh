@@ -17,9 +17,8 @@ constexpr float kLn2 = 0.6931471805599453f;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// One lane of the warp, always the same one.  (Behind it the compiler knows that a tensor instruction is issued once for the
-// warp and keeps its operands in uniform registers; behind a test of the lane's number it moves them there one by one, some
-// 150 cycles for each instruction of a starved warp.)
+// One lane of the warp, always the same one.  (Behind it a tensor instruction takes a warp that gets few issue slots some 40
+// cycles, behind a test of the lane's number 150: measured in the tile kernels.)
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r)::"memory");

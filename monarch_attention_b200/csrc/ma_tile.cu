@@ -16,10 +16,11 @@
 // the waits of one CTA (loads, tensor pipe, tensor memory) are covered by the other CTAs of the SM instead of by a
 // pipeline of specialised warps.  What bounds it: at 256 keys the latency of the row passes, with eight row warps on an SM.  A
 // right-factor tile of 128 x 256 takes its CTA 10600 cycles (16 heads of 65536 tokens: 8192 tiles on 296 places in 155 us; the
-// stages of two iterations 155, 253, 183, 159), 5300 of the SM's per tile; the pipe of exponentials and conversions, 32 lanes a
-// clock, needs 2048, and the row passes alone take 2950 with eight warps on an SM.  (Tensor instructions behind a test of the
-// lane's number instead of an elected lane: 163, 258, 196, 165.  Rows stored by their threads instead of by TMA took 1700 cycles of that chain; launching the next stage early, by programmatic dependent launch,
-// cost the running stage its instruction cache: 18000 cycles for the first tile instead of 9000.)
+// stages of two iterations 155-157, 253, 183-186, 159), 5300 of the SM's per tile; the pipe of exponentials and conversions, 32
+// lanes a clock, needs 2048, and the row passes alone take 2950 with eight warps on an SM.  (Tensor instructions behind a test of
+// the lane's number instead of an elected lane: 163, 258, 196, 165.  Rows stored by their threads instead of by TMA took 1700
+// cycles of that chain; launching the next stage early, by programmatic dependent launch, cost the running stage its instruction
+// cache: 18000 cycles for the first tile instead of 9000.)
 //
 // Rounding points are the reference's: S is rounded to storage before the softmax, P is normalised in fp32 and then
 // rounded.  Ragged ends, padding and masks: rows that do not exist are zero-filled by TMA (or by hand, where a column's

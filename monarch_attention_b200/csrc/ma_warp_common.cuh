@@ -104,7 +104,9 @@ __device__ __forceinline__ int reduce_rows(float (&v)[N], int lane) {
 // column for every piece were 300 of 2530 (16 x 16 x 72) for each tile (67.3 instead of 72 us for 128 heads of 256 x 72, three
 // iterations).  16-bit types, whose rows are one or two lines: one piece after the other, with row, column chunk, token index
 // and source offset carried along by additions only; shared rows were slower there (64 x 12 heads of 197 x 64: 39.1 instead of
-// 37.1 us; 8 x 16 of 2025 x 80: 115 instead of 107).
+// 37.1 us; 8 x 16 of 2025 x 80: 115 instead of 107).  Together with store_rows' stores from fragments, which the backward kernels
+// share, a training step in fp32 went from 479 to 461 us (4 x 12 heads of 1024 x 64, three iterations) and from 1058 to 996 (2 x 12
+// of 4096 x 64, two).
 template <typename T, int CHUNKS>  // CHUNKS: 16-byte pieces of a padded row
 __device__ __forceinline__ void load_rows(T* tile, int pitch, int rows, int rpad, int width, const T* base, int n0,
                                           int nstep, int n_limit, long long row_stride, int tid, int nthreads,
