@@ -234,8 +234,8 @@ int run_forward(const ma_b200_problem* p, int mask_type, void* workspace, size_t
   const bool flow = L.kernel == MA_B200_KERNEL_TILE && ma::flow_supported(g);
   if (L.kernel != MA_B200_KERNEL_WARP_MMA && L.kernel != MA_B200_KERNEL_TF32X3 && L.kernel != MA_B200_KERNEL_HEAD_RESIDENT &&
       L.kernel != MA_B200_KERNEL_HEAD_FUSED && L.kernel != MA_B200_KERNEL_TILE) {
-    ce = cudaMemsetAsync(ws + L.status, 0, L.ar - L.status, stream);
-    if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemsetAsync(status, counters)");
+    ce = ma::launch_clear(ws + L.status, L.ar - L.status, stream);
+    if (ce != cudaSuccess) return cuda_fail(ce, "clearing status and counters");
   }
   int* counters = reinterpret_cast<int*>(ws + L.counters);
 

@@ -288,7 +288,8 @@ constexpr int right_ctas(int element_bytes, int KP, bool with_v) { return KP == 
 template <typename T, int KP, int DP, bool WITH_V>
 __global__ void __launch_bounds__(2 * KP, right_ctas(sizeof(T), KP, WITH_V)) backward_right_kernel(const BackwardArgs a) {
   constexpr int PITCH = DP + 8, PP = KP + 8;
-  stage_begin();
+  if (!a.first) dependents_may_start();
+  grid_wait();
   extern __shared__ __align__(16) uint8_t smem[];
   const Geometry& g = a.g;
   const int eh = blockIdx.y, e = eh / g.H, h = eh - e * g.H, m = blockIdx.x;
@@ -476,7 +477,7 @@ cudaError_t backward_launch(const BackwardArgs& a, BackwardStage st, size_t* sme
   if (const cudaError_t e = allow_dynamic_smem(fn, smem); e != cudaSuccess) return e;
   const int rows = right ? g.B : g.M;
   void* args[] = {(void*)&a};
-  return launch_stage(fn, dim3(right ? g.M : g.B, g.E * g.H), dim3(2 * ((rows + 15) & ~15)), args, smem, true, stream);
+  return launch_kernel(fn, dim3(right ? g.M : g.B, g.E * g.H), dim3(2 * ((rows + 15) & ~15)), args, smem, stream);
 }
 
 template <typename T, int KP>

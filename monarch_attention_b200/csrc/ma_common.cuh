@@ -115,27 +115,38 @@ __device__ __forceinline__ bool mask_lets(const Geometry& g, int e, int n) {
   }
 }
 
-// A stage kernel of a call after the first one: its CTAs are brought up under the tail of the stage before, and each waits at
-// its start (stage_begin) until that stage is complete and its stores are visible.  (256 fp32 tokens, two launches: 15.4 to
-// 13.3 us; six launches 84 to 75.  The tcgen05 tile kernels lost by it: their early CTAs took instruction fetch from the
-// running stage.)
-inline cudaError_t launch_stage(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, bool overlap, cudaStream_t stream) {
-  if (!overlap) return cudaLaunchKernel(fn, grid, block, args, smem, stream);
+// Kernels are launched with programmatic dependence on whatever precedes them in the stream, another library's kernel included:
+// the GPU then prepares the launch while that kernel ends, and the kernel waits at its start (grid_wait), before it touches
+// memory, until everything before it is complete and visible.  A plain launch costs more than its work here: launches of a
+// kernel that spins for t us follow one another every ceil((t + 1) / 2.05) * 2.05 us (3 us: 6.15, 10: 12.30, 16: 18.43), with
+// the dependence every t + 0.55 (148 or 768 CTAs, with and without clusters, 0 to 200 KB of shared memory).
+// A stage kernel that another stage follows also lets that one's CTAs come up at once (stage_begin), under its own tail: 256 fp32
+// tokens, two launches, 15.4 to 13.3 us; six launches 84 to 75.  The last kernel of a call does not, so that a small grid behind
+// it finds all SMs free and spreads evenly, nor do the tcgen05 tile kernels: their early CTAs took instruction fetch from the
+// running stage.
+// A kernel that allocates tensor memory does so behind grid_wait, or behind a kernel that has passed its own: a kernel in front
+// that lets its dependents start before it has tensor memory of its own would wait for ours, and we for its end.
+inline cudaError_t launch_kernel(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t stream, int cluster = 1) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attrs[2] = {};
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = cluster;
+  attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void stage_begin() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  dependents_may_start();
+  grid_wait();
 }
 
 // Host-side launchers implemented by the kernel translation units.
@@ -193,6 +204,8 @@ cudaError_t launch_tile_stage(const Geometry& g, int dtype, StageKind kind, bool
 // Their single-launch form, all stages of a call, for block size and count up to 128 (ma_flow.cu); counters: (E*H, 2T)
 // zeroed ints, as the status block.  wait_expiry (self-test): the first stage is left out, so that the waits for it run out.
 bool flow_supported(const Geometry& g);
+// `bytes` from p on to zero, rounded up to whole pieces of 16; p on a 16-byte boundary.
+cudaError_t launch_clear(void* p, size_t bytes, cudaStream_t stream);
 cudaError_t launch_flow(const Geometry& g, int dtype, int* counters, int* host_status, bool wait_expiry, cudaStream_t stream);
 // Code of a bounded device-side wait that gave up on `device` since the last poll (0 = none); reads a mapped
 // host word, so it needs no synchronisation.

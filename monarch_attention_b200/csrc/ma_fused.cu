@@ -226,6 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1) fused_kernel(const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_wait();  // (launch_clear has passed its own, so nothing in front still wants tensor memory)
 
   // Only the planner walks the item schedule.  It leaves a four-word descriptor per item in a small
   // ring (written before the arrive that hands the item to the issuer, whose arrive on the item's
@@ -954,7 +955,21 @@ cudaError_t launch_fused(const TcPlan* plan, const Geometry& g, int* counters, i
   const int total = (stage_end - stage_begin) * (g.N / kTile) * g.E * g.H;
   const int grid = total < sms ? total : sms;
   void* params[] = {(void*)&plan->maps, (void*)&g, (void*)&a};
-  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), params, kSmemBytes, stream);
+  // cooperative: a CTA waits for items of all the others; and under the tail of what clears the counters (the attribute saves
+  // less beside a cooperative launch: its starts stay on the grid of 2.05 us)
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attrs[2] = {};
+  attrs[0].id = cudaLaunchAttributeCooperative;
+  attrs[0].val.cooperative = 1;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelExC(&cfg, fn, params);
 }
 
 }  // namespace ma

@@ -145,9 +145,11 @@ __global__ void __launch_bounds__(kTileThreads, tile_ctas(NK))
     for (int i = 0; i < kTileBars; ++i) mbar_init(bar(i), i == kBarP || i == kBarE ? kRows : 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (args.clear && blockIdx.x == 0) *g.status = 0;
   }
+  grid_wait();
+  if (args.clear && blockIdx.x == 0 && tid == 0) *g.status = 0;
   if (warp == 4) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(stage + kOffAux + 3 * 256 * 4 + 8 * kTileBars + 8),
                  "r"(kCols)
                  : "memory");
@@ -588,7 +590,7 @@ cudaError_t launch_tile_typed(const Geometry& g, const TileMaps& maps, const Til
   if (const cudaError_t e = allow_dynamic_smem(fn, smem); e != cudaSuccess) return e;
   // one CTA for each place on the GPU; it takes tiles round-robin and loads the next one under the present one
   void* params[] = {(void*)&maps, (void*)&g, (void*)&args};
-  return cudaLaunchKernel(fn, dim3(std::min(args.total, sm_count() * tile_ctas(NK))), dim3(kTileThreads), params, smem, stream);
+  return launch_kernel(fn, dim3(std::min(args.total, sm_count() * tile_ctas(NK))), dim3(kTileThreads), params, smem, stream);
 }
 
 template <typename T, int NK>
