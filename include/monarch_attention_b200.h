@@ -277,6 +277,13 @@ MA_B200_API int ma_b200_forward_host(const ma_b200_problem* p, int heads_per_chu
  * copy, as above; results arrive in call order. */
 MA_B200_API int ma_b200_forward_host_streamed(const ma_b200_problem* p, int heads_per_chunk, void* device_scratch,
                                               size_t scratch_bytes, void* stream);
+/* Both forms (streamed: 0 or 1) with chunks for heads of a few kilobytes, whose copies take less than the 25 us that a chunk
+ * costs the host: with heads_per_chunk >= H a chunk takes up to elements_per_chunk whole batch elements, and the chunks at
+ * the end shrink no further than to least_heads heads.  With elements_per_chunk = least_heads = 1 they are the forms above. */
+MA_B200_API size_t ma_b200_host_scratch_bytes_grouped(const ma_b200_problem* p, int heads_per_chunk, int elements_per_chunk);
+MA_B200_API int ma_b200_forward_host_grouped(const ma_b200_problem* p, int heads_per_chunk, int elements_per_chunk,
+                                             int least_heads, int streamed, void* device_scratch, size_t scratch_bytes,
+                                             void* stream);
 MA_B200_API const char* ma_b200_host_last_error(void);
 
 MA_B200_API int32_t ma_b200_abi_version(void);

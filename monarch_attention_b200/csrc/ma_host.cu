@@ -5,12 +5,14 @@
 // independent in every stage, so the call is cut into chunks of a few heads and pipelined over
 // three streams owned by the library -
 //     copy-in : H2D q, k, v of chunk i+1
-//     compute : ma_b200_forward on chunk i (device staging buffers, E = 1, H = heads of the chunk; the kernel family of
-//               the whole call, so that the result has the bits of one call on device tensors)
+//     compute : ma_b200_forward on chunk i (device staging buffers, some heads of one batch element or several whole
+//               elements; the kernel family of the whole call, so that the result has the bits of one call on device tensors)
 //     copy-out: D2H result of chunk i-1
 // - with three staging slots in caller-provided device memory and events between the streams.
 // PCIe is full duplex, so the steady state is bound by the larger copy direction alone; the chunks of
 // the last batch element shrink towards the end so that little is left exposed after the last copy-in.
+// A chunk costs the host 25 us (three copies, a launch, a copy and the events between them), and the copy engines some
+// more, so small chunks are bound by that: heads of a few kilobytes are grouped across batch elements (the caller says how many).
 // The whole pipeline is queued from one host thread without waiting for the GPU; on return the
 // caller's stream has been made to wait for the last copy.
 #include <mutex>
@@ -43,25 +45,28 @@ size_t elem_size(int dtype) { return dtype == MA_B200_F32 ? 4 : 2; }
 
 struct HostLayout {
   int hc;                                // heads per chunk (clamped to H)
+  int ec;                                // batch elements per chunk (more than one only with all heads)
   size_t qk_bytes, v_bytes;              // one staging tensor of a slot
   size_t slot_bytes, mask_off, mask_bytes, ws_off, ws_bytes, total;
 };
 
 // 0 on success; fills the layout of the device scratch for this problem.
-int host_layout(const ma_b200_problem* p, int heads_per_chunk, HostLayout* L, std::string* err) {
+int host_layout(const ma_b200_problem* p, int heads_per_chunk, int elements_per_chunk, HostLayout* L, std::string* err) {
   if (p == nullptr) { *err = "problem is null"; return MA_B200_INVALID_ARGUMENT; }
   if (heads_per_chunk < 1) { *err = "heads_per_chunk must be at least 1"; return MA_B200_INVALID_ARGUMENT; }
+  if (elements_per_chunk < 1) { *err = "elements_per_chunk must be at least 1"; return MA_B200_INVALID_ARGUMENT; }
   if (p->E < 1 || p->H < 1 || p->N < 1 || p->D < 1 || p->Dv < 1) { *err = "E, H, N, D, Dv must be positive"; return MA_B200_INVALID_ARGUMENT; }
   L->hc = heads_per_chunk < p->H ? heads_per_chunk : p->H;
-  L->qk_bytes = round_up((size_t)L->hc * p->N * p->D * elem_size(p->qk_dtype));
-  L->v_bytes = round_up((size_t)L->hc * p->N * p->Dv * elem_size(p->v_dtype));
+  L->ec = L->hc < p->H ? 1 : elements_per_chunk < p->E ? elements_per_chunk : p->E;
+  L->qk_bytes = round_up((size_t)L->ec * L->hc * p->N * p->D * elem_size(p->qk_dtype));
+  L->v_bytes = round_up((size_t)L->ec * L->hc * p->N * p->Dv * elem_size(p->v_dtype));
   L->slot_bytes = 2 * L->qk_bytes + 2 * L->v_bytes;  // q, k, v, result
   L->mask_off = kSlots * L->slot_bytes;
   L->mask_bytes = p->mask != nullptr ? round_up((size_t)p->E * p->N) : 0;
   L->ws_off = L->mask_off + L->mask_bytes;
   // workspace of the largest chunk problem (pointers are not looked at by the size query)
   ma_b200_problem sub = *p;
-  sub.E = 1;
+  sub.E = L->ec;
   sub.H = L->hc;
   sub.q.ptr = sub.k.ptr = sub.v.ptr = sub.out.ptr = nullptr;
   sub.q.stride_e = sub.k.stride_e = (int64_t)L->hc * p->N * p->D;
@@ -101,11 +106,22 @@ int get_pipes(Pipes** out, std::string* err) {
   return MA_B200_OK;
 }
 
-// Copies `heads` heads of one batch element between a strided host tensor and a dense staging
-// buffer (heads, N, W).  One copy when the heads are dense in host memory, one (pitched) copy per
+// Copies `heads` heads of each of `elements` batch elements between a strided host tensor and a dense staging
+// buffer (elements, heads, N, W).  One copy where they are dense in host memory, one (pitched) copy per
 // head otherwise.
-cudaError_t copy_heads(void* dev, const ma_b200_tensor& host, int e, int h0, int heads, int N, int W, size_t es,
+cudaError_t copy_heads(void* dev, const ma_b200_tensor& host, int e, int elements, int h0, int heads, int N, int W, size_t es,
                        bool to_device, cudaStream_t s) {
+  if (elements > 1) {
+    if (host.stride_n == W && host.stride_h == (int64_t)N * W && host.stride_e == heads * host.stride_h) {
+      heads *= elements;  // (whole elements: h0 is 0)
+    } else {
+      for (int i = 0; i < elements; ++i)
+        if (const cudaError_t ce = copy_heads(static_cast<char*>(dev) + (size_t)i * heads * N * W * es, host, e + i, 1, h0, heads, N, W, es, to_device, s);
+            ce != cudaSuccess)
+          return ce;
+      return cudaSuccess;
+    }
+  }
   char* hbase = static_cast<char*>(const_cast<void*>(host.ptr)) + ((int64_t)e * host.stride_e + (int64_t)h0 * host.stride_h) * (int64_t)es;
   const bool rows_dense = host.stride_n == W;
   const bool heads_dense = rows_dense && (heads == 1 || host.stride_h == (int64_t)N * W);
@@ -135,19 +151,27 @@ extern "C" {
 
 MA_B200_API const char* ma_b200_host_last_error(void) { return g_host_error.c_str(); }
 
-MA_B200_API size_t ma_b200_host_scratch_bytes(const ma_b200_problem* p, int heads_per_chunk) {
+MA_B200_API size_t ma_b200_host_scratch_bytes_grouped(const ma_b200_problem* p, int heads_per_chunk, int elements_per_chunk) {
   HostLayout L;
   g_host_error.clear();
-  if (host_layout(p, heads_per_chunk, &L, &g_host_error) != MA_B200_OK) return 0;
+  if (host_layout(p, heads_per_chunk, elements_per_chunk, &L, &g_host_error) != MA_B200_OK) return 0;
   return L.total;
 }
 
-static int forward_host_impl(const ma_b200_problem* p, int heads_per_chunk, void* device_scratch, size_t scratch_bytes,
-                             void* stream_v, bool streamed) {
+MA_B200_API size_t ma_b200_host_scratch_bytes(const ma_b200_problem* p, int heads_per_chunk) {
+  return ma_b200_host_scratch_bytes_grouped(p, heads_per_chunk, 1);
+}
+
+MA_B200_API int ma_b200_forward_host_grouped(const ma_b200_problem* p, int heads_per_chunk, int elements_per_chunk, int least_heads,
+                                             int streamed, void* device_scratch, size_t scratch_bytes, void* stream_v) {
   g_host_error.clear();
   HostLayout L;
-  int rc = host_layout(p, heads_per_chunk, &L, &g_host_error);
+  int rc = host_layout(p, heads_per_chunk, elements_per_chunk, &L, &g_host_error);
   if (rc != MA_B200_OK) return rc;
+  if (least_heads < 1) {
+    g_host_error = "least_heads must be at least 1";
+    return MA_B200_INVALID_ARGUMENT;
+  }
   if (p->q.ptr == nullptr || p->k.ptr == nullptr || p->v.ptr == nullptr || p->out.ptr == nullptr) {
     g_host_error = "q, k, v and out must be host pointers";
     return MA_B200_INVALID_ARGUMENT;
@@ -178,7 +202,7 @@ static int forward_host_impl(const ma_b200_problem* p, int heads_per_chunk, void
   // copying out, provided that call used the scratch in the same way (same slots: the per-slot events then
   // order every reuse); anything else is ordered after what the caller has already queued on its stream,
   // which includes the end of the previous call.
-  const bool overlap = streamed && P->last_scratch == device_scratch && P->last_slot_bytes == L.slot_bytes &&
+  const bool overlap = streamed != 0 && P->last_scratch == device_scratch && P->last_slot_bytes == L.slot_bytes &&
                        P->last_total == L.total;
   P->last_scratch = device_scratch;
   P->last_slot_bytes = L.slot_bytes;
@@ -204,15 +228,16 @@ static int forward_host_impl(const ma_b200_problem* p, int heads_per_chunk, void
   }
 
   int i = 0, kernel = 0;  // one kernel family for all chunks: the one of a call on device tensors with all heads
-  for (int e = 0; e < p->E; ++e) {
+  for (int e = 0, ne = 1; e < p->E; e += ne) {
+    ne = L.ec < p->E - e ? L.ec : p->E - e;
     int nh = 0;
     for (int h0 = 0; h0 < p->H; h0 += nh, ++i) {
       // Chunks of hc heads, except that the last batch element tapers off (each chunk at most half of
-      // what is left): once the last copy-in has landed, only the kernels and the copy-out of the last
-      // chunk are still to come, and nothing overlaps them.
+      // what is left, and at least least_heads): once the last copy-in has landed, only the kernels and the copy-out of the
+      // last chunk are still to come, and nothing overlaps them.
       const int left = p->H - h0;
       nh = left < L.hc ? left : L.hc;
-      if (e == p->E - 1 && nh > 1 && nh > left / 2) nh = left / 2 > 1 ? left / 2 : 1;
+      if (ne == 1 && e == p->E - 1 && nh > least_heads && nh > left / 2) nh = left / 2 > least_heads ? left / 2 : least_heads;
       const int slot = i % kSlots;
       char* sq = base + (size_t)slot * L.slot_bytes;
       char* sk = sq + L.qk_bytes;
@@ -220,15 +245,15 @@ static int forward_host_impl(const ma_b200_problem* p, int heads_per_chunk, void
       char* so = sv + L.v_bytes;
       // copy in: the kernels of the chunk that used this slot last have read q, k, v
       if (i >= kSlots || overlap) MA_TRY(cudaStreamWaitEvent(P->in, P->computed[slot], 0), "wait(in, computed)");
-      MA_TRY(copy_heads(sq, p->q, e, h0, nh, p->N, p->D, es_qk, true, P->in), "H2D q");
-      MA_TRY(copy_heads(sk, p->k, e, h0, nh, p->N, p->D, es_qk, true, P->in), "H2D k");
-      MA_TRY(copy_heads(sv, p->v, e, h0, nh, p->N, p->Dv, es_v, true, P->in), "H2D v");
+      MA_TRY(copy_heads(sq, p->q, e, ne, h0, nh, p->N, p->D, es_qk, true, P->in), "H2D q");
+      MA_TRY(copy_heads(sk, p->k, e, ne, h0, nh, p->N, p->D, es_qk, true, P->in), "H2D k");
+      MA_TRY(copy_heads(sv, p->v, e, ne, h0, nh, p->N, p->Dv, es_v, true, P->in), "H2D v");
       MA_TRY(cudaEventRecord(P->loaded[slot], P->in), "record(loaded)");
       // compute: inputs landed, and the previous result of this slot has left it
       MA_TRY(cudaStreamWaitEvent(P->comp, P->loaded[slot], 0), "wait(comp, loaded)");
       if (i >= kSlots || overlap) MA_TRY(cudaStreamWaitEvent(P->comp, P->stored[slot], 0), "wait(comp, stored)");
       ma_b200_problem sub = *p;
-      sub.E = 1;
+      sub.E = ne;
       sub.H = nh;
       sub.q = {sq, (int64_t)nh * p->N * p->D, (int64_t)p->N * p->D, p->D};
       sub.k = {sk, (int64_t)nh * p->N * p->D, (int64_t)p->N * p->D, p->D};
@@ -246,7 +271,7 @@ static int forward_host_impl(const ma_b200_problem* p, int heads_per_chunk, void
       MA_TRY(cudaEventRecord(P->computed[slot], P->comp), "record(computed)");
       // copy out
       MA_TRY(cudaStreamWaitEvent(P->out, P->computed[slot], 0), "wait(out, computed)");
-      MA_TRY(copy_heads(so, p->out, e, h0, nh, p->N, p->Dv, es_v, false, P->out), "D2H result");
+      MA_TRY(copy_heads(so, p->out, e, ne, h0, nh, p->N, p->Dv, es_v, false, P->out), "D2H result");
       MA_TRY(cudaEventRecord(P->stored[slot], P->out), "record(stored)");
     }
   }
@@ -261,12 +286,12 @@ static int forward_host_impl(const ma_b200_problem* p, int heads_per_chunk, void
 
 MA_B200_API int ma_b200_forward_host(const ma_b200_problem* p, int heads_per_chunk, void* device_scratch,
                                      size_t scratch_bytes, void* stream_v) {
-  return forward_host_impl(p, heads_per_chunk, device_scratch, scratch_bytes, stream_v, false);
+  return ma_b200_forward_host_grouped(p, heads_per_chunk, 1, 1, 0, device_scratch, scratch_bytes, stream_v);
 }
 
 MA_B200_API int ma_b200_forward_host_streamed(const ma_b200_problem* p, int heads_per_chunk, void* device_scratch,
                                               size_t scratch_bytes, void* stream_v) {
-  return forward_host_impl(p, heads_per_chunk, device_scratch, scratch_bytes, stream_v, true);
+  return ma_b200_forward_host_grouped(p, heads_per_chunk, 1, 1, 1, device_scratch, scratch_bytes, stream_v);
 }
 
 }  // extern "C"

@@ -20,6 +20,22 @@ from .monarch_attention import _check_device_free_inputs, make_problem
 
 _scratch: dict[int, Tensor] = {}
 
+# Least bytes of one tensor in a chunk.  A chunk of a few heads whatever their size was bound by what it costs the host and the
+# copy engines to start.  Measured (us, 8 heads a chunk / chunks of at least 1, 2, 4, 8 MB): 52 x 12 heads of 93 x 64 in fp32
+# 2940 / 1284, 1105, 1092, 1084 (copying in alone 810); 5 x 12 of 769 x 64 650 / 591, 517, 466, 497; 16 x 16 of 512 x 64 1621 /
+# 1426, 1274, 1176, 1170; 8 of 8192 x 64, whose chunks are larger anyway, 699 / 679, 684, 667, 684.
+CHUNK_BYTES = 4 << 20
+
+
+def group_chunks(E: int, H: int, head_bytes: int, heads_per_chunk: int) -> tuple[int, int, int]:
+    """(heads per chunk, batch elements per chunk, least heads of a chunk at the end): a chunk of less than CHUNK_BYTES of one
+    tensor grows to that, over whole batch elements where it has all their heads, and shrinks no further than to half of it at
+    the end."""
+    room = -(-CHUNK_BYTES // head_bytes)
+    heads = min(H, max(heads_per_chunk, room))
+    elements = min(E, max(1, room // H)) if heads == H else 1
+    return heads, elements, max(1, room // 2)
+
 
 def plan_chunks(E: int, H: int, heads_per_chunk: int) -> list[tuple[int, int, int]]:
     """(batch index, first head, number of heads) of every chunk, in the order the library runs them."""
@@ -49,8 +65,8 @@ def monarch_attention_b200_host(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tens
     q, k, v: CPU tensors (E, H, N, D) / (E, H, N, Dv) with unit inner stride; pinned for overlap.
     out:     optional CPU tensor (E, H, N, Dv) to receive the result (pinned for overlap).
     device:  CUDA device to run on (default: the current one).
-    heads_per_chunk: heads per pipeline chunk (the last chunks are smaller: each at most half of what is
-             left); 8 measured best for 16 heads of N = 16384 (2.20 ms per call against 2.60 ms unpipelined;
+    heads_per_chunk: heads per pipeline chunk (more where that is less than ``CHUNK_BYTES`` of a tensor, see ``group_chunks``; the
+             last chunks are smaller: each at most half of what is left); 8 measured best for 16 heads of N = 16384 (2.20 ms per call against 2.60 ms unpipelined;
              4 gives 2.23 ms, 2 loses again to per-chunk start-up).
     wait:    block until the result is in ``out``; with ``wait=False`` the current stream has been made
              to wait for the last copy instead, and the caller synchronises it before reading ``out``
@@ -82,7 +98,8 @@ def monarch_attention_b200_host(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tens
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     prob = make_problem(q, k, v, out, mask, T, B, pre_pad, kernel)
     with torch.cuda.device(device):
-        need = lib.ma_b200_host_scratch_bytes(C.byref(prob), heads_per_chunk)
+        heads, elements, least = group_chunks(E, H, N * max(q.shape[-1], Dv) * q.element_size(), heads_per_chunk)
+        need = lib.ma_b200_host_scratch_bytes_grouped(C.byref(prob), heads, elements)
         if need == 0:
             raise ValueError(lib.ma_b200_host_last_error().decode())
         idx = device.index if device.index is not None else torch.cuda.current_device()
@@ -91,8 +108,8 @@ def monarch_attention_b200_host(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tens
             torch.cuda.synchronize(device)  # an earlier call may still be using the old scratch
             scratch = _scratch[idx] = torch.empty(need, dtype=torch.uint8, device=device)
         stream = torch.cuda.current_stream(device)
-        entry = lib.ma_b200_forward_host_streamed if streamed else lib.ma_b200_forward_host
-        rc = entry(C.byref(prob), heads_per_chunk, scratch.data_ptr(), scratch.numel(), stream.cuda_stream)
+        rc = lib.ma_b200_forward_host_grouped(C.byref(prob), heads, elements, least, int(streamed), scratch.data_ptr(),
+                                              scratch.numel(), stream.cuda_stream)
         if rc != 0:
             _cabi.raise_for_status(rc, lib.ma_b200_host_last_error().decode())
         if wait:
