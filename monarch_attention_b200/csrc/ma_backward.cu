@@ -86,9 +86,35 @@ __device__ __forceinline__ void zero_acc(float (&o)[DP / 8][4]) {
   for (int nt = 0; nt < DP / 8; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
 }
 
-// Rows r of a fp32 accumulator array: row_ptr(r) is the row or nullptr.  add: memory += o, else memory = o.
+// Rows of a fp32 accumulator array as fragments.  All loads are asked for before the first one is used: addition by addition, with
+// the stores between them, each waited for memory by itself: forward and backward of 4 x 12 heads of 1024 x 64, three iterations, 197 ->
+// 172 us (the kernels that add, 21-24 -> 15-17); 2 x 12 of 4096 411 -> 361; 8 x 16 of 256 x 72 in fp32 291 -> 250.
+template <int DP>
+struct RowsF32 {
+  float2 v[2][DP / 8];
+  template <typename RowFn>
+  __device__ __forceinline__ void load(RowFn row_ptr, int D, int lane) {
+    const int gq = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const float* p = row_ptr(gq + 8 * half);
+#pragma unroll
+      for (int nt = 0; nt < DP / 8; ++nt) {
+        const int c = nt * 8 + 2 * t;
+        v[half][nt] = p != nullptr && c < D ? *reinterpret_cast<const float2*>(p + c) : make_float2(0.f, 0.f);
+      }
+    }
+  }
+  __device__ __forceinline__ void add_to(float (&o)[DP / 8][4]) const {
+#pragma unroll
+    for (int nt = 0; nt < DP / 8; ++nt) {
+      o[nt][0] += v[0][nt].x; o[nt][1] += v[0][nt].y;
+      o[nt][2] += v[1][nt].x; o[nt][3] += v[1][nt].y;
+    }
+  }
+};
 template <int DP, typename RowFn>
-__device__ __forceinline__ void update_rows_f32(float (&o)[DP / 8][4], RowFn row_ptr, int D, int lane, bool add) {
+__device__ __forceinline__ void store_rows_f32(const float (&o)[DP / 8][4], RowFn row_ptr, int D, int lane) {
   const int gq = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
@@ -97,32 +123,22 @@ __device__ __forceinline__ void update_rows_f32(float (&o)[DP / 8][4], RowFn row
 #pragma unroll
     for (int nt = 0; nt < DP / 8; ++nt) {
       const int c = nt * 8 + 2 * t;
-      if (c >= D) continue;
-      float2 x = make_float2(o[nt][2 * half], o[nt][2 * half + 1]);
-      if (add) {
-        const float2 y = *reinterpret_cast<const float2*>(p + c);
-        x.x += y.x; x.y += y.y;
-      }
-      *reinterpret_cast<float2*>(p + c) = x;
+      if (c < D) *reinterpret_cast<float2*>(p + c) = make_float2(o[nt][2 * half], o[nt][2 * half + 1]);
     }
   }
 }
 // o += rows of a fp32 array.
 template <int DP, typename RowFn>
 __device__ __forceinline__ void add_rows_f32(float (&o)[DP / 8][4], RowFn row_ptr, int D, int lane) {
-  const int gq = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const float* p = row_ptr(gq + 8 * half);
-    if (p == nullptr) continue;
-#pragma unroll
-    for (int nt = 0; nt < DP / 8; ++nt) {
-      const int c = nt * 8 + 2 * t;
-      if (c >= D) continue;
-      const float2 y = *reinterpret_cast<const float2*>(p + c);
-      o[nt][2 * half] += y.x; o[nt][2 * half + 1] += y.y;
-    }
-  }
+  RowsF32<DP> rows;
+  rows.load(row_ptr, D, lane);
+  rows.add_to(o);
+}
+// add: memory += o, else memory = o.
+template <int DP, typename RowFn>
+__device__ __forceinline__ void update_rows_f32(float (&o)[DP / 8][4], RowFn row_ptr, int D, int lane, bool add) {
+  if (add) add_rows_f32<DP>(o, row_ptr, D, lane);
+  store_rows_f32<DP>(o, row_ptr, D, lane);
 }
 
 template <typename T>
@@ -279,10 +295,10 @@ constexpr size_t right_elems(bool with_v, int RP) {
 // registers; with V seven, which is what shared memory holds at width 64 (28.3 KB each), so that no register is given up for more.
 // 8 x 16 heads of 1024 tokens at width 72, two iterations: 334.7 us with ten for both kinds (the instances with V then
 // spill at widths above 64), 332.2 left to the compiler, 331.4 as it is; 4 x 12 heads at width 64, three iterations: 193.0, 193.7, 192.0.
-// The fp32 instances for up to 64 keys take all 255 registers and spill (460 bytes a thread at width 64, 776 with V; 860 and
-// 1076 at width 80): the logit and factor rows of a warp alone are 2 x 32 registers, their split halves as many again.  They are
-// still worth having: forward and backward of 2 x 12 heads of 4096 tokens, two iterations, 1074 us against 3425 by tensor
-// operations at width 64, 1605 against 4009 at width 80.
+// The fp32 instances for up to 64 keys take all 255 registers and spill (264 bytes a thread at width 64, 736 with V; 864 and
+// 1240 at width 80): the logit and factor rows of a warp alone are 2 x 32 registers, their split halves as many again.  They are
+// still worth having: forward and backward of 2 x 12 heads of 4096 tokens, two iterations, 973 us against 3425 by tensor
+// operations at width 64, 1506 against 4009 at width 80.
 constexpr int right_ctas(int element_bytes, int KP, bool with_v) { return KP == 32 && element_bytes == 2 ? (with_v ? 7 : 10) : 1; }
 
 template <typename T, int KP, int DP, bool WITH_V>
