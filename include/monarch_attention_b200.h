@@ -66,7 +66,7 @@ enum { MA_B200_F32 = 0, MA_B200_BF16 = 1, MA_B200_F16 = 2 };
  *   TF32X3         the WARP_MMA stage kernels on f32 tensors, block size and block count up to 128,
  *                  D <= 80 (multiple of 8): every operand split into two tf32 parts (2T launches)
  *   HEAD_RESIDENT  16-bit inputs, block size and block count up to 32, D <= 80 (multiple of 8): one CTA
- *                  or cluster per head, all stages in one launch, the head's state on chip where it fits
+ *                  or a few per head, all stages in one launch, the head's state on chip where it fits
  *   TILE           tcgen05 stage kernels, one 128-row tile per CTA: 16-bit inputs, block size and block count
  *                  up to 256, D <= 64 (multiple of 8), masks and padding (one launch up to 128, else 2T) */
 enum {

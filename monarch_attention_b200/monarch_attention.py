@@ -148,7 +148,7 @@ class MonarchAttention(nn.Module):
     ``impl`` selects the kernel family: "b200" (default: the library picks by shape, type and number of
     heads), "b200-tcgen05" (fused, one launch), "b200-tcgen05-staged" (same kernel, one launch per stage),
     "b200-tile" (tcgen05 tile kernels, one launch up to blocks of 128), "b200-head-resident" (small blocks: one
-    CTA or cluster per head, all stages), "b200-head-fused" (the same, one iteration only), "b200-warp-mma"
+    CTA or a few per head, all stages), "b200-head-fused" (the same, one iteration only), "b200-warp-mma"
     (warp-level tensor-core kernels), "b200-tf32x3" (the same on fp32 tensors) or "b200-generic".  The reference's
     "torch" and "triton" implementations are not part of this library; asking for an
     unknown name raises ``ValueError`` exactly as the reference does.

@@ -11,7 +11,7 @@ SHAPES = [  # one for each way a call is launched
     ((1, 4, 200 * 180, 64, 200, 2), torch.bfloat16),  # tile kernels, a launch per stage
     ((1, 4, 4096, 64, 64, 2), torch.bfloat16),        # fused kernel
     ((64, 12, 197, 64, 15, 2), torch.bfloat16),       # head-resident kernel
-    ((2, 3, 197, 64, 15, 2), torch.bfloat16),         # ... in clusters
+    ((2, 3, 197, 64, 15, 2), torch.bfloat16),         # ... in parts
     ((1, 2, 40 * 60, 80, 40, 2), torch.bfloat16),     # warp-level kernels
     ((2, 12, 256, 64, 16, 2), torch.float32),         # fp32 tensor path, one launch
     ((20, 8, 256, 64, 16, 2), torch.float32),         # ... a launch per stage
