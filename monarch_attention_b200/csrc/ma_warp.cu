@@ -23,5 +23,24 @@
 // Explicit launcher templates are declared before use in ma_warp_kernels.inc and defined in
 // ma_warp_wide.inc, so the public entry points have to come last.
 #include "ma_warp_kernels.inc"
-#include "ma_warp_head.inc"
 #include "ma_warp_wide.inc"
+
+namespace ma {
+
+cudaError_t launch_warp_stage_f32(const Geometry& g, StageKind kind, bool first, cudaStream_t stream);  // ma_warp_f32.cu
+
+bool warp_supported(const Geometry& g, int qk_dtype, int v_dtype, const char** why) {
+  if (qk_dtype != v_dtype || (qk_dtype != MA_B200_BF16 && qk_dtype != MA_B200_F16)) {
+    *why = "needs bf16 or f16 for q, k and v";
+    return false;
+  }
+  return tile_shape_supported(g, 8, why);
+}
+
+cudaError_t launch_warp_stage(const Geometry& g, int qk_dtype, StageKind kind, bool first, cudaStream_t stream) {
+  if (qk_dtype == MA_B200_BF16) return launch_warp_kp<__nv_bfloat16>(g, kind, first, stream);
+  if (qk_dtype == MA_B200_F32) return launch_warp_stage_f32(g, kind, first, stream);
+  return launch_warp_kp<__half>(g, kind, first, stream);
+}
+
+}  // namespace ma
