@@ -145,12 +145,14 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, long long he
   // list fewer waits, 16.5 / 18.5 and 18.5 / 18.7 at 0.9, 20.4 / 19.3 and 21.3 / 20.8 at 1.7, 22.7 / 21.8 and 24.9 / 24.7 at 2.6: the
   // line at 2 was drawn before the roles of the tile kernels were split, and takes up to 5 % too long between 1 and 2.
   const bool few_tiles = tc_ok && heads * p->N / 64 <= (long long)ma::sm_count() * (p->num_steps == 1 ? 4 : 11);
-  // Head widths other than 64 and 72 have one tile size for both kinds of stage in the head-resident kernel: with one side of
+  // Head widths other than 32, 64, 72 and 80 have one tile size for both kinds of stage in the head-resident kernel: with one side of
   // up to 16 beside a longer one the warp-level kernels pad less, and win once the heads no longer fit the SMs in one round.
-  // Measured (us, head-resident / warp-level; widths 32 to 80, blocks of 8 x 20 to 16 x 24, one and two iterations), 10 x 30 x 80
-  // with two: 33 / 37 at 148 heads, 60 / 39 at 160, 88 / 62 at 300, 124 / 115 at 592; 10 x 30 x 32 with one: 13 / 16, 21 / 17,
-  // 32 / 23, 39 / 37.  (Against the rule: width 32 and many heads with two iterations, 61 / 78 at 592 heads of 16 x 24.)
-  const bool lopsided = (g.B <= 16) != (g.M <= 16) && g.D != 64 && g.D != 72 && heads > ma::sm_count();
+  // Measured before 32 and 80 had tiles of their own (us, head-resident / warp-level; blocks of 8 x 20 to 16 x 24, one and two
+  // iterations), 10 x 30 x 80 with two: 33 / 37 at 148 heads, 60 / 39 at 160, 88 / 62 at 300, 124 / 115 at 592; 10 x 30 x 32 with one:
+  // 13 / 16, 21 / 17, 32 / 23, 39 / 37.  With tiles of their own, head-resident / warp-level: 10 x 30 x 32 with one 10.7 / 14.6 at 160, 17.5 /
+  // 19.7 at 300, 25.2 / 34.2 at 592, 16 x 24 x 32 with two 18.1 / 27.9, 28.6 / 42.1, 38.7 / 74.8; 10 x 30 x 80 with two 34.0 / 37.4, 54.6 /
+  // 58.8, 77.0 / 112.  Width 80 is still on the other side of this line, since parts of calls are held to the family it gives.
+  const bool lopsided = (g.B <= 16) != (g.M <= 16) && g.D != 32 && g.D != 64 && g.D != 72 && heads > ma::sm_count();
   if (p->kernel == MA_B200_KERNEL_AUTO)
     *kernel = few_tiles ? MA_B200_KERNEL_TCGEN05
               : resident_ok && !lopsided ? MA_B200_KERNEL_HEAD_RESIDENT
