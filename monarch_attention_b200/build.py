@@ -19,7 +19,7 @@ LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libmonarch_attention_b200.so")
 NATIVE_PATH = os.path.join(PKG, "_native.so")
 NATIVE_SOURCE = "ma_torch.cpp"
-SOURCES = ["ma_api.cu", "ma_generic.cu", "ma_tc.cu", "ma_fused.cu", "ma_warp.cu", "ma_warp_f32.cu", "ma_head.cu", "ma_head_f16.cu", "ma_tile.cu", "ma_flow.cu", "ma_flow_f16.cu", "ma_backward.cu", "ma_backward_f16.cu", "ma_backward_f32.cu", "ma_noalloc.cu", "ma_host.cu"]
+SOURCES = ["ma_api.cu", "ma_generic.cu", "ma_tc.cu", "ma_fused.cu", "ma_warp.cu", "ma_warp_f32.cu", "ma_head.cu", "ma_head_f16.cu", "ma_head_states.cu", "ma_head_states_f16.cu", "ma_tile.cu", "ma_flow.cu", "ma_flow_f16.cu", "ma_backward.cu", "ma_backward_f16.cu", "ma_backward_f32.cu", "ma_noalloc.cu", "ma_host.cu"]
 HEADERS = ["ma_common.cuh", "ma_tile_common.cuh", "ma_flow.inc", "ma_head.inc", "ma_backward.inc", "ma_warp_common.cuh", "ma_warp_kernels.inc", "ma_warp_head.inc", "ma_warp_wide.inc", "ma_sm100.cuh", "ma_tc_plan.cuh", os.path.join("..", "..", "include", "monarch_attention_b200.h")]
 
 NVCC_FLAGS = [

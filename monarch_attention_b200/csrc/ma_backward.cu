@@ -76,11 +76,17 @@ cudaError_t launch_backward(const Geometry& g0, int dtype, const View4& dz, cons
   cudaError_t e;
   const int T = g0.T;
   // ---- the forward stages, every iteration's state kept ---------------------------------------------------
-  for (int t = 0; t < T; ++t) {
-    if ((e = launch_warp_stage(at_iteration(t, t), dtype, t == T - 1 ? kStageRightWithV : kStageRight, t == 0, stream)) != cudaSuccess)
-      return e;
-    if (t < T - 1)
-      if ((e = launch_warp_stage(at_iteration(t + 1, t), dtype, kStageLeft, false, stream)) != cudaSuccess) return e;
+  if (head_states_pay(g0, dtype)) {
+    const BackwardStates s{ws + L.al, ws + L.ar, ws + L.y, reinterpret_cast<float*>(ws + L.cl), reinterpret_cast<float*>(ws + L.cr),
+                           (long long)L.mat, (long long)L.vec};
+    if ((e = launch_head_states(at_iteration(0, 0), dtype, s, stream)) != cudaSuccess) return e;
+  } else {
+    for (int t = 0; t < T; ++t) {
+      if ((e = launch_warp_stage(at_iteration(t, t), dtype, t == T - 1 ? kStageRightWithV : kStageRight, t == 0, stream)) != cudaSuccess)
+        return e;
+      if (t < T - 1)
+        if ((e = launch_warp_stage(at_iteration(t + 1, t), dtype, kStageLeft, false, stream)) != cudaSuccess) return e;
+    }
   }
   // ---- and back -------------------------------------------------------------------------------------------
   BackwardArgs a{};

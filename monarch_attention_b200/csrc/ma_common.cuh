@@ -190,6 +190,16 @@ void tc_plan_destroy(TcPlan* plan);
 // All stages of the fp32 tensor path (TF32X3) in one launch, for block size and count up to 32 (ma_warp_head.inc).
 bool head_f32_pays(const Geometry& g);
 cudaError_t launch_head_f32(const Geometry& g, cudaStream_t stream);
+// The stage inputs of the backward pass in one launch, where the head-resident kernel has tiles for the shape (ma_head_states.cu): al
+// and y (EH, B, M, D), ar (EH, M, B, D), cl (EH, B, M), cr (EH, M, B); those of an iteration `mat` and `vec` bytes behind those of
+// the one before, ar and cr from the second iteration on.
+struct BackwardStates {
+  char *al, *ar, *y;
+  float *cl, *cr;
+  long long mat, vec;
+};
+bool head_states_pay(const Geometry& g, int dtype);
+cudaError_t launch_head_states(const Geometry& g, int dtype, const BackwardStates& s, cudaStream_t stream);
 // Persistent fused kernel: stages [stage_begin, stage_end) of the 2T stages in one cooperative launch.
 size_t fused_counter_bytes(const Geometry& g);
 // (spin_limit: iterations of the dependency wait before it gives up, 0 = default; for the wait-expiry self-test.)
