@@ -526,8 +526,8 @@ def run_ours(args, rank, world, local):
     t_tensor = flops / (peaks["bf16_tflops"] * 1e12)
     t_hbm = nbytes / (peaks["hbm_gbs"] * 1e9)
     achieved_tflops = flops / (ms_step * 1e-3) / 1e12
-    # kernels of a step: one a stage, or one for all of them, before which the tile kernels have one that clears their counters
-    launches = n_stage if not one_launch else 2 if kernel == _cabi.KERNEL_TILE else 1
+    # kernels of a step: one a stage, or one for all of them, before which the kernels that count have one that clears their counters
+    launches = n_stage if not one_launch else 2 if kernel in (_cabi.KERNEL_TILE, _cabi.KERNEL_TCGEN05) else 1
     roofline = {
         "bound": "tensor" if t_tensor >= t_hbm else "hbm",
         "achieved": achieved_tflops, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
