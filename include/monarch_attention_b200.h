@@ -174,7 +174,8 @@ typedef struct ma_b200_gradients {
 /* Enqueue the backward pass of `p` on `stream` (p->out and p->kernel are ignored).  The stage inputs are recomputed
  * from q, k, v, so nothing has to be kept from the forward call.  Takes the problems of the WARP_MMA and TF32X3
  * kernels with block size and block count up to 128 (64 in fp32); ma_b200_backward_workspace_bytes returns 0 for others (the caller
- * then differentiates a recomputation).
+ * then differentiates a recomputation).  The gradients of a head do not depend on what else is in the call: parts of a call
+ * (batch or head shards, micro-batches) have the bits of the whole.
  * reference: autograd through ma/ma_torch.py:10-108, which is how the reference trains. */
 MA_B200_API size_t ma_b200_backward_workspace_bytes(const ma_b200_problem* p);
 MA_B200_API int ma_b200_backward(const ma_b200_problem* p, const ma_b200_gradients* g, void* workspace,
