@@ -135,7 +135,8 @@ MA_B200_API int ma_b200_workspace_layout_of(const ma_b200_problem* p, ma_b200_wo
  * one part (with NULL pointers alignment is taken for granted); only whether mask is NULL is looked at. */
 MA_B200_API int ma_b200_kernel_of_part(const ma_b200_problem* part, int64_t heads);
 
-/* Enqueue the forward pass on `stream` (a cudaStream_t / CUstream; NULL = default stream).
+/* Enqueue the forward pass on `stream` (a cudaStream_t / CUstream; NULL = default stream).  `out` may be q, k or v itself (same
+ * pointer and strides).
  * reference: monarch_attention_torch, ma/ma_torch.py:65-108. */
 MA_B200_API int ma_b200_forward(const ma_b200_problem* p, void* workspace, size_t workspace_bytes, void* stream);
 
