@@ -25,13 +25,14 @@ _scratch: dict[int, Tensor] = {}
 # 2940 / 1284, 1105, 1092, 1084 (copying in alone 810); 5 x 12 of 769 x 64 650 / 591, 517, 466, 497; 16 x 16 of 512 x 64 1621 /
 # 1426, 1274, 1176, 1170; 8 of 8192 x 64, whose chunks are larger anyway, 699 / 679, 684, 667, 684.
 CHUNK_BYTES = 4 << 20
+HEADS_PER_CHUNK = 8
 
 
-def group_chunks(E: int, H: int, head_bytes: int, heads_per_chunk: int) -> tuple[int, int, int]:
-    """(heads per chunk, batch elements per chunk, least heads of a chunk at the end): a chunk of less than CHUNK_BYTES of one
-    tensor grows to that, over whole batch elements where it has all their heads, and shrinks no further than to half of it at
-    the end."""
-    room = -(-CHUNK_BYTES // head_bytes)
+def group_chunks(E: int, H: int, head_bytes: int, heads_per_chunk: int, chunk_bytes: int | None = None) -> tuple[int, int, int]:
+    """(heads per chunk, batch elements per chunk, least heads of a chunk at the end): a chunk of less than ``chunk_bytes``
+    (default CHUNK_BYTES) of one tensor grows to that, over whole batch elements where it has all their heads, and shrinks no
+    further than to half of it at the end.  With 0 it is ``heads_per_chunk`` heads of one batch element."""
+    room = -(-(CHUNK_BYTES if chunk_bytes is None else chunk_bytes) // head_bytes)
     heads = min(H, max(heads_per_chunk, room))
     elements = min(E, max(1, room // H)) if heads == H else 1
     return heads, elements, max(1, room // 2)
@@ -58,16 +59,19 @@ def plan_chunks(E: int, H: int, heads_per_chunk: int) -> list[tuple[int, int, in
 
 def monarch_attention_b200_host(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tensor | None, T: int, B: int,
                                 pre_pad: bool, *, out: Tensor | None = None, device=None,
-                                heads_per_chunk: int = 8, wait: bool = True, streamed: bool = False,
-                                kernel: int = _cabi.KERNEL_AUTO) -> Tensor:
+                                heads_per_chunk: int = HEADS_PER_CHUNK, wait: bool = True, streamed: bool = False,
+                                kernel: int = _cabi.KERNEL_AUTO, chunk_bytes: int | None = None) -> Tensor:
     """Same computation as ``monarch_attention_b200`` for q, k, v (and the result) in host memory.
 
     q, k, v: CPU tensors (E, H, N, D) / (E, H, N, Dv) with unit inner stride; pinned for overlap.
     out:     optional CPU tensor (E, H, N, Dv) to receive the result (pinned for overlap).
     device:  CUDA device to run on (default: the current one).
-    heads_per_chunk: heads per pipeline chunk (more where that is less than ``CHUNK_BYTES`` of a tensor, see ``group_chunks``; the
-             last chunks are smaller: each at most half of what is left); 8 measured best for 16 heads of N = 16384 (2.20 ms per call against 2.60 ms unpipelined;
-             4 gives 2.23 ms, 2 loses again to per-chunk start-up).
+    heads_per_chunk: most heads in a pipeline chunk (the last chunks are smaller: each at most half of what is left), and with that
+             the device scratch: three chunks and the workspace of one; 8 measured best for 16 heads of N = 16384 (2.20 ms per call
+             against 2.60 ms unpipelined; 4 gives 2.23 ms, 2 loses again to per-chunk start-up).  Small heads are
+             grouped beyond the default 8, see ``chunk_bytes``.
+    chunk_bytes: chunks of less than this of a tensor grow to it, over batch elements too (``group_chunks``).  Default: ``CHUNK_BYTES``
+             with the default heads_per_chunk, 0 (never) with any other.
     wait:    block until the result is in ``out``; with ``wait=False`` the current stream has been made
              to wait for the last copy instead, and the caller synchronises it before reading ``out``
              (and keeps q, k, v, the mask and ``out`` alive until then).
@@ -81,6 +85,10 @@ def monarch_attention_b200_host(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tens
         raise ValueError("monarch_attention_b200_host takes host tensors; use monarch_attention_b200 for device ones")
     if heads_per_chunk < 1:
         raise ValueError("heads_per_chunk must be at least 1")
+    if chunk_bytes is None:
+        chunk_bytes = CHUNK_BYTES if heads_per_chunk == HEADS_PER_CHUNK else 0
+    elif chunk_bytes < 0:
+        raise ValueError("chunk_bytes must not be negative")
     E, H, N, _ = q.shape
     Dv = v.shape[-1]
     if out is None:
@@ -98,7 +106,7 @@ def monarch_attention_b200_host(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tens
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     prob = make_problem(q, k, v, out, mask, T, B, pre_pad, kernel)
     with torch.cuda.device(device):
-        heads, elements, least = group_chunks(E, H, N * max(q.shape[-1], Dv) * q.element_size(), heads_per_chunk)
+        heads, elements, least = group_chunks(E, H, N * max(q.shape[-1], Dv) * q.element_size(), heads_per_chunk, chunk_bytes)
         need = lib.ma_b200_host_scratch_bytes_grouped(C.byref(prob), heads, elements)
         if need == 0:
             raise ValueError(lib.ma_b200_host_last_error().decode())

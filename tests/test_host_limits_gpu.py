@@ -1,0 +1,58 @@
+"""What bounds the device scratch of the host entry point: heads_per_chunk, and chunk_bytes where heads are small."""
+import ctypes as C
+
+import pytest
+import torch
+
+
+def test_no_grouping_with_chunk_bytes_of_zero():
+    from monarch_attention_b200.host_pipeline import group_chunks
+    assert group_chunks(9, 4, 64, 2, 0) == (2, 1, 1) and group_chunks(9, 4, 64, 7, 0) == (4, 1, 1)
+    assert group_chunks(9, 4, 64, 2, 64 * 12) == (4, 3, 6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("asked,per_chunk,elements", [({"heads_per_chunk": 1}, 1, 1), ({"heads_per_chunk": 5}, 5, 1), ({}, 12, 6),
+                                                      ({"chunk_bytes": 0}, 8, 1), ({"heads_per_chunk": 2, "chunk_bytes": 30 * 1000}, 5, 1)])
+def test_scratch_is_what_was_asked_for(monkeypatch, asked, per_chunk, elements):
+    import monarch_attention_b200 as ma
+    from monarch_attention_b200 import _cabi, host_pipeline
+    from monarch_attention_b200.monarch_attention import make_problem
+    monkeypatch.setattr(host_pipeline, "_scratch", {})
+    g = torch.Generator().manual_seed(3)
+    q, k, v = (torch.randn(6, 12, 50, 64, generator=g).to(torch.bfloat16).pin_memory() for _ in range(3))
+    dev = torch.device("cuda:0")
+    out = ma.monarch_attention_b200_host(q, k, v, None, 2, 8, False, **asked)
+    assert torch.equal(out, ma.MonarchAttention(8, 2, "post")(q.to(dev), k.to(dev), v.to(dev)).cpu())
+    need = _cabi.load().ma_b200_host_scratch_bytes_grouped(C.byref(make_problem(q, k, v, out, None, 2, 8, False)), per_chunk, elements)
+    assert host_pipeline._scratch[0].numel() == need
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("chunk", [1, 3 * 4 * 50 * 64 * 2, 4 << 20])  # of one head, of three elements (the last ragged), all at once
+@pytest.mark.parametrize("layout", ["heads", "tokens", "gaps"])
+@pytest.mark.parametrize("masked", [False, True])
+def test_chunks_over_elements_return_the_bits_of_one_device_call(chunk, layout, masked):
+    import monarch_attention_b200 as ma
+    E, H, N, D, B, T = 8, 4, 50, 64, 8, 2
+    g = torch.Generator().manual_seed(chunk % 89)
+
+    def host():
+        t = torch.randn(E, H, N, D, generator=g).to(torch.bfloat16)
+        if layout == "tokens":
+            return t.permute(0, 2, 1, 3).contiguous().pin_memory().permute(0, 2, 1, 3)
+        if layout == "gaps":  # elements that do not follow one another
+            whole = torch.zeros(E, H + 1, N, D, dtype=t.dtype).pin_memory()
+            whole[:, :H] = t
+            return whole[:, :H]
+        return t.pin_memory()
+
+    q, k, v = host(), host(), host()
+    m = torch.rand(E, N, generator=g) > 0.3 if masked else None
+    dev = torch.device("cuda:0")
+    want = ma.MonarchAttention(B, T, "pre")(q.to(dev), k.to(dev), v.to(dev), None if m is None else m.to(dev)).cpu()
+    out = host()
+    for streamed in (False, True, True):
+        out.zero_()
+        ma.monarch_attention_b200_host(q, k, v, m, T, B, True, out=out, heads_per_chunk=1, chunk_bytes=chunk, streamed=streamed)
+        assert torch.equal(out.contiguous().view(torch.int16), want.contiguous().view(torch.int16))
