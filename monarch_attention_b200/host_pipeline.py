@@ -103,8 +103,10 @@ def monarch_attention_b200_host(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tens
     if attn_mask is not None:
         mask = attn_mask.view(torch.uint8) if attn_mask.dtype == torch.bool else (attn_mask != 0).view(torch.uint8)
         mask = mask if mask.stride(-1) == 1 else mask.contiguous()
-    device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     prob = make_problem(q, k, v, out, mask, T, B, pre_pad, kernel)
+    if lib.ma_b200_host_scratch_bytes(C.byref(prob), heads_per_chunk) == 0:  # (says what is wrong with the problem, if anything is)
+        raise ValueError(lib.ma_b200_host_last_error().decode())
+    device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     with torch.cuda.device(device):
         heads, elements, least = group_chunks(E, H, N * max(q.shape[-1], Dv) * q.element_size(), heads_per_chunk, chunk_bytes)
         need = lib.ma_b200_host_scratch_bytes_grouped(C.byref(prob), heads, elements)

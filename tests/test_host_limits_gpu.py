@@ -11,6 +11,16 @@ def test_no_grouping_with_chunk_bytes_of_zero():
     assert group_chunks(9, 4, 64, 2, 64 * 12) == (4, 3, 6)
 
 
+@pytest.mark.parametrize("shape,T,B,heads,error", [((1, 2, 8, 0), 1, 4, 8, ValueError), ((2, 3, 8, 16), 0, 4, 8, ValueError),
+                                                   ((2, 3, 8, 16), 1, 0, 8, ValueError), ((2, 3, 8, 16), 1, 4, 0, ValueError),
+                                                   ((2, 3, 8, 16), 1, 4, 8.0, C.ArgumentError)])
+def test_refused_before_a_gpu_is_touched(shape, T, B, heads, error):
+    from monarch_attention_b200 import monarch_attention_b200_host
+    t = torch.zeros(shape)
+    with pytest.raises(error):
+        monarch_attention_b200_host(t, t, t, None, T, B, False, out=torch.zeros(shape), device="cuda:0", heads_per_chunk=heads)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("asked,per_chunk,elements", [({"heads_per_chunk": 1}, 1, 1), ({"heads_per_chunk": 5}, 5, 1), ({}, 12, 6),
                                                       ({"chunk_bytes": 0}, 8, 1), ({"heads_per_chunk": 2, "chunk_bytes": 30 * 1000}, 5, 1)])
