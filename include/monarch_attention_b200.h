@@ -280,12 +280,17 @@ MA_B200_API int ma_b200_forward_host(const ma_b200_problem* p, int heads_per_chu
 MA_B200_API int ma_b200_forward_host_streamed(const ma_b200_problem* p, int heads_per_chunk, void* device_scratch,
                                               size_t scratch_bytes, void* stream);
 /* Both forms (streamed: 0 or 1) with chunks for heads of a few kilobytes, whose copies take less than the 25 us that a chunk
- * costs the host: with heads_per_chunk >= H a chunk takes up to elements_per_chunk whole batch elements, and the chunks at
- * the end shrink no further than to least_heads heads.  With elements_per_chunk = least_heads = 1 they are the forms above. */
+ * costs the host: with heads_per_chunk >= H a chunk takes up to elements_per_chunk whole batch elements, the chunks of an element
+ * before the last are as even as they can be, and at the end no chunk is cut to fewer than least_heads heads (what such a cut
+ * leaves may be fewer).  With elements_per_chunk = least_heads = 1 they are the forms above. */
 MA_B200_API size_t ma_b200_host_scratch_bytes_grouped(const ma_b200_problem* p, int heads_per_chunk, int elements_per_chunk);
 MA_B200_API int ma_b200_forward_host_grouped(const ma_b200_problem* p, int heads_per_chunk, int elements_per_chunk,
                                              int least_heads, int streamed, void* device_scratch, size_t scratch_bytes,
                                              void* stream);
+/* The chunks of a call in the order they are run, as (batch element, first head, number of heads, which may reach over whole
+ * elements) in chunks[0 .. 3 * min(capacity, their number)); returns their number, -1 on an invalid argument. */
+MA_B200_API int ma_b200_host_chunk_plan(int E, int H, int heads_per_chunk, int elements_per_chunk, int least_heads, int32_t* chunks,
+                                        int capacity);
 MA_B200_API const char* ma_b200_host_last_error(void);
 
 MA_B200_API int32_t ma_b200_abi_version(void);

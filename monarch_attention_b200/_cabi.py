@@ -26,7 +26,7 @@ EXPORTS = (
     "ma_b200_device_status", "ma_b200_status_string", "ma_b200_last_error", "ma_b200_abi_version",
     "ma_b200_forward_static_scratch", "ma_b200_static_scratch_bytes", "ma_b200_static_scratch_last_error",
     "ma_b200_host_scratch_bytes", "ma_b200_forward_host", "ma_b200_forward_host_streamed", "ma_b200_host_last_error",
-    "ma_b200_host_scratch_bytes_grouped", "ma_b200_forward_host_grouped",
+    "ma_b200_host_scratch_bytes_grouped", "ma_b200_forward_host_grouped", "ma_b200_host_chunk_plan",
     "ma_b200_poll_device_status", "ma_b200_selftest_wait_expiry", "ma_b200_selftest_generic_general_form",
     "ma_b200_backward_workspace_bytes", "ma_b200_backward", "ma_b200_forward_typed_mask", "ma_b200_backward_typed_mask",
 )
@@ -118,6 +118,8 @@ def load() -> C.CDLL:
     lib.ma_b200_host_scratch_bytes_grouped.restype = C.c_size_t
     lib.ma_b200_forward_host_grouped.argtypes = [pp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_size_t, C.c_void_p]
     lib.ma_b200_forward_host_grouped.restype = C.c_int
+    lib.ma_b200_host_chunk_plan.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int32), C.c_int]
+    lib.ma_b200_host_chunk_plan.restype = C.c_int
     lib.ma_b200_host_last_error.argtypes = []
     lib.ma_b200_host_last_error.restype = C.c_char_p
     if lib.ma_b200_abi_version() != ABI_VERSION:

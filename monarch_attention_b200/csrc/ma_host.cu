@@ -43,6 +43,11 @@ thread_local std::string g_host_error;
 size_t round_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 size_t elem_size(int dtype) { return dtype == MA_B200_F32 ? 4 : 2; }
 
+void clamp_chunk(int E, int H, int heads, int elements, int* hc, int* ec) {
+  *hc = heads < H ? heads : H;
+  *ec = *hc < H ? 1 : elements < E ? elements : E;
+}
+
 struct HostLayout {
   int hc;                                // heads per chunk (clamped to H)
   int ec;                                // batch elements per chunk (more than one only with all heads)
@@ -56,8 +61,7 @@ int host_layout(const ma_b200_problem* p, int heads_per_chunk, int elements_per_
   if (heads_per_chunk < 1) { *err = "heads_per_chunk must be at least 1"; return MA_B200_INVALID_ARGUMENT; }
   if (elements_per_chunk < 1) { *err = "elements_per_chunk must be at least 1"; return MA_B200_INVALID_ARGUMENT; }
   if (p->E < 1 || p->H < 1 || p->N < 1 || p->D < 1 || p->Dv < 1) { *err = "E, H, N, D, Dv must be positive"; return MA_B200_INVALID_ARGUMENT; }
-  L->hc = heads_per_chunk < p->H ? heads_per_chunk : p->H;
-  L->ec = L->hc < p->H ? 1 : elements_per_chunk < p->E ? elements_per_chunk : p->E;
+  clamp_chunk(p->E, p->H, heads_per_chunk, elements_per_chunk, &L->hc, &L->ec);
   L->qk_bytes = round_up((size_t)L->ec * L->hc * p->N * p->D * elem_size(p->qk_dtype));
   L->v_bytes = round_up((size_t)L->ec * L->hc * p->N * p->Dv * elem_size(p->v_dtype));
   L->slot_bytes = 2 * L->qk_bytes + 2 * L->v_bytes;  // q, k, v, result
@@ -104,6 +108,32 @@ int get_pipes(Pipes** out, std::string* err) {
   }
   *out = &P;
   return MA_B200_OK;
+}
+
+// Heads [h0, h0 + heads) of the batch elements [e, e + elements); more than one element only with all their heads.
+struct Chunk {
+  int e, elements, h0, heads;
+};
+int ceil_div(int a, int b) { return (a + b - 1) / b; }
+// The chunk behind `c` (e = E: there is none); c = {0, 0, 0, 0} gives the first.  Chunks of `ec` elements where they have all hc = H
+// heads, else of hc heads.  The last batch element tapers off when it is by itself: a chunk is cut to half of what is left, but not below
+// `least` heads; what that leaves may be fewer.  Small heads (least > 1): chunks of an earlier element are as even as they can be.
+// Measured, us: 6 x 20 heads of 2300 x 64 in chunks of 15 and 5 / 10 and 10 2476 / 2419, 3 x 16 15 and 1 / 8 and 8 1032 / 1002, 2 x 24 of 1500
+// x 64 714 / 699.  Not so at the end, where a small last chunk leaves little to copy out: 12 heads of 3000 x 64 in chunks of 6, 5, 1 / 6, 6
+// 378 / 396, 16 of 2300 x 64 8, 7, 1 / 8, 8 389 / 402; nor over elements: 52 x 12 of 93 x 64 in fp32 14, 14, 14, 10 / 13, 13, 13, 13 1077 / 1119.
+Chunk next_chunk(const Chunk& c, int E, int H, int hc, int ec, int least) {
+  const bool more = c.elements == 1 && c.h0 + c.heads < H;  // of the same element
+  Chunk n{more ? c.e : c.e + c.elements, 1, more ? c.h0 + c.heads : 0, 0};
+  if (n.e >= E) return n;
+  const int left = H - n.h0;
+  if (ec > 1) n.elements = ec < E - n.e ? ec : E - n.e;
+  if (n.elements > 1 || n.e < E - 1) {
+    n.heads = least > 1 ? ceil_div(left, ceil_div(left, hc)) : left < hc ? left : hc;
+  } else {
+    n.heads = left < hc ? left : hc;
+    if (n.heads > least && n.heads > left / 2) n.heads = left / 2 > least ? left / 2 : least;
+  }
+  return n;
 }
 
 // Copies `heads` heads of each of `elements` batch elements between a strided host tensor and a dense staging
@@ -160,6 +190,25 @@ MA_B200_API size_t ma_b200_host_scratch_bytes_grouped(const ma_b200_problem* p, 
 
 MA_B200_API size_t ma_b200_host_scratch_bytes(const ma_b200_problem* p, int heads_per_chunk) {
   return ma_b200_host_scratch_bytes_grouped(p, heads_per_chunk, 1);
+}
+
+MA_B200_API int ma_b200_host_chunk_plan(int E, int H, int heads_per_chunk, int elements_per_chunk, int least_heads, int32_t* chunks,
+                                        int capacity) {
+  g_host_error.clear();
+  if (E < 0 || H < 0 || heads_per_chunk < 1 || elements_per_chunk < 1 || least_heads < 1) {
+    g_host_error = "E and H must not be negative, heads_per_chunk, elements_per_chunk and least_heads at least 1";
+    return -1;
+  }
+  int hc, ec, n = 0;
+  clamp_chunk(E, H, heads_per_chunk, elements_per_chunk, &hc, &ec);
+  if (E == 0 || H == 0) return 0;
+  for (Chunk c = next_chunk({0, 0, 0, 0}, E, H, hc, ec, least_heads); c.e < E; c = next_chunk(c, E, H, hc, ec, least_heads), ++n)
+    if (n < capacity) {
+      chunks[3 * n] = c.e;
+      chunks[3 * n + 1] = c.h0;
+      chunks[3 * n + 2] = c.elements * c.heads;
+    }
+  return n;
 }
 
 MA_B200_API int ma_b200_forward_host_grouped(const ma_b200_problem* p, int heads_per_chunk, int elements_per_chunk, int least_heads,
@@ -228,52 +277,44 @@ MA_B200_API int ma_b200_forward_host_grouped(const ma_b200_problem* p, int heads
   }
 
   int i = 0, kernel = 0;  // one kernel family for all chunks: the one of a call on device tensors with all heads
-  for (int e = 0, ne = 1; e < p->E; e += ne) {
-    ne = L.ec < p->E - e ? L.ec : p->E - e;
-    int nh = 0;
-    for (int h0 = 0; h0 < p->H; h0 += nh, ++i) {
-      // Chunks of hc heads, except that the last batch element tapers off (each chunk at most half of
-      // what is left, and at least least_heads): once the last copy-in has landed, only the kernels and the copy-out of the
-      // last chunk are still to come, and nothing overlaps them.
-      const int left = p->H - h0;
-      nh = left < L.hc ? left : L.hc;
-      if (ne == 1 && e == p->E - 1 && nh > least_heads && nh > left / 2) nh = left / 2 > least_heads ? left / 2 : least_heads;
-      const int slot = i % kSlots;
-      char* sq = base + (size_t)slot * L.slot_bytes;
-      char* sk = sq + L.qk_bytes;
-      char* sv = sk + L.qk_bytes;
-      char* so = sv + L.v_bytes;
-      // copy in: the kernels of the chunk that used this slot last have read q, k, v
-      if (i >= kSlots || overlap) MA_TRY(cudaStreamWaitEvent(P->in, P->computed[slot], 0), "wait(in, computed)");
-      MA_TRY(copy_heads(sq, p->q, e, ne, h0, nh, p->N, p->D, es_qk, true, P->in), "H2D q");
-      MA_TRY(copy_heads(sk, p->k, e, ne, h0, nh, p->N, p->D, es_qk, true, P->in), "H2D k");
-      MA_TRY(copy_heads(sv, p->v, e, ne, h0, nh, p->N, p->Dv, es_v, true, P->in), "H2D v");
-      MA_TRY(cudaEventRecord(P->loaded[slot], P->in), "record(loaded)");
-      // compute: inputs landed, and the previous result of this slot has left it
-      MA_TRY(cudaStreamWaitEvent(P->comp, P->loaded[slot], 0), "wait(comp, loaded)");
-      if (i >= kSlots || overlap) MA_TRY(cudaStreamWaitEvent(P->comp, P->stored[slot], 0), "wait(comp, stored)");
-      ma_b200_problem sub = *p;
-      sub.E = ne;
-      sub.H = nh;
-      sub.q = {sq, (int64_t)nh * p->N * p->D, (int64_t)p->N * p->D, p->D};
-      sub.k = {sk, (int64_t)nh * p->N * p->D, (int64_t)p->N * p->D, p->D};
-      sub.v = {sv, (int64_t)nh * p->N * p->Dv, (int64_t)p->N * p->Dv, p->Dv};
-      sub.out = {so, (int64_t)nh * p->N * p->Dv, (int64_t)p->N * p->Dv, p->Dv};
-      sub.mask = mask_dev != nullptr ? mask_dev + (size_t)e * p->N : nullptr;
-      sub.mask_stride_e = mask_dev != nullptr ? p->N : 0;
-      if (kernel == 0) kernel = ma_b200_kernel_of_part(&sub, (int64_t)p->E * p->H);
-      if (kernel != 0) sub.kernel = kernel;  // (0: ma_b200_forward says why)
-      rc = ma_b200_forward(&sub, base + L.ws_off, L.ws_bytes, P->comp);
-      if (rc != MA_B200_OK) {
-        g_host_error = std::string("chunk forward: ") + ma_b200_last_error();
-        return rc;
-      }
-      MA_TRY(cudaEventRecord(P->computed[slot], P->comp), "record(computed)");
-      // copy out
-      MA_TRY(cudaStreamWaitEvent(P->out, P->computed[slot], 0), "wait(out, computed)");
-      MA_TRY(copy_heads(so, p->out, e, ne, h0, nh, p->N, p->Dv, es_v, false, P->out), "D2H result");
-      MA_TRY(cudaEventRecord(P->stored[slot], P->out), "record(stored)");
+  auto behind = [&](const Chunk& c) { return next_chunk(c, p->E, p->H, L.hc, L.ec, least_heads); };
+  for (Chunk c = behind({0, 0, 0, 0}); c.e < p->E; c = behind(c), ++i) {
+    const int e = c.e, ne = c.elements, h0 = c.h0, nh = c.heads;
+    const int slot = i % kSlots;
+    char* sq = base + (size_t)slot * L.slot_bytes;
+    char* sk = sq + L.qk_bytes;
+    char* sv = sk + L.qk_bytes;
+    char* so = sv + L.v_bytes;
+    // copy in: the kernels of the chunk that used this slot last have read q, k, v
+    if (i >= kSlots || overlap) MA_TRY(cudaStreamWaitEvent(P->in, P->computed[slot], 0), "wait(in, computed)");
+    MA_TRY(copy_heads(sq, p->q, e, ne, h0, nh, p->N, p->D, es_qk, true, P->in), "H2D q");
+    MA_TRY(copy_heads(sk, p->k, e, ne, h0, nh, p->N, p->D, es_qk, true, P->in), "H2D k");
+    MA_TRY(copy_heads(sv, p->v, e, ne, h0, nh, p->N, p->Dv, es_v, true, P->in), "H2D v");
+    MA_TRY(cudaEventRecord(P->loaded[slot], P->in), "record(loaded)");
+    // compute: inputs landed, and the previous result of this slot has left it
+    MA_TRY(cudaStreamWaitEvent(P->comp, P->loaded[slot], 0), "wait(comp, loaded)");
+    if (i >= kSlots || overlap) MA_TRY(cudaStreamWaitEvent(P->comp, P->stored[slot], 0), "wait(comp, stored)");
+    ma_b200_problem sub = *p;
+    sub.E = ne;
+    sub.H = nh;
+    sub.q = {sq, (int64_t)nh * p->N * p->D, (int64_t)p->N * p->D, p->D};
+    sub.k = {sk, (int64_t)nh * p->N * p->D, (int64_t)p->N * p->D, p->D};
+    sub.v = {sv, (int64_t)nh * p->N * p->Dv, (int64_t)p->N * p->Dv, p->Dv};
+    sub.out = {so, (int64_t)nh * p->N * p->Dv, (int64_t)p->N * p->Dv, p->Dv};
+    sub.mask = mask_dev != nullptr ? mask_dev + (size_t)e * p->N : nullptr;
+    sub.mask_stride_e = mask_dev != nullptr ? p->N : 0;
+    if (kernel == 0) kernel = ma_b200_kernel_of_part(&sub, (int64_t)p->E * p->H);
+    if (kernel != 0) sub.kernel = kernel;  // (0: ma_b200_forward says why)
+    rc = ma_b200_forward(&sub, base + L.ws_off, L.ws_bytes, P->comp);
+    if (rc != MA_B200_OK) {
+      g_host_error = std::string("chunk forward: ") + ma_b200_last_error();
+      return rc;
     }
+    MA_TRY(cudaEventRecord(P->computed[slot], P->comp), "record(computed)");
+    // copy out
+    MA_TRY(cudaStreamWaitEvent(P->out, P->computed[slot], 0), "wait(out, computed)");
+    MA_TRY(copy_heads(so, p->out, e, ne, h0, nh, p->N, p->Dv, es_v, false, P->out), "D2H result");
+    MA_TRY(cudaEventRecord(P->stored[slot], P->out), "record(stored)");
   }
   // the caller's stream continues once the last kernel and the last copy are done
   MA_TRY(cudaEventRecord(P->done_comp, P->comp), "record(done_comp)");

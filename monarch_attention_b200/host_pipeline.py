@@ -30,31 +30,26 @@ HEADS_PER_CHUNK = 8
 
 def group_chunks(E: int, H: int, head_bytes: int, heads_per_chunk: int, chunk_bytes: int | None = None) -> tuple[int, int, int]:
     """(heads per chunk, batch elements per chunk, least heads of a chunk at the end): a chunk of less than ``chunk_bytes``
-    (default CHUNK_BYTES) of one tensor grows to that, over whole batch elements where it has all their heads, and shrinks no
-    further than to half of it at the end.  With 0 it is ``heads_per_chunk`` heads of one batch element."""
+    (default CHUNK_BYTES) of one tensor grows to that, over whole batch elements where it has all their heads, and is not cut to
+    fewer than half of it at the end.  With 0 it is ``heads_per_chunk`` heads of one batch element."""
     room = -(-(CHUNK_BYTES if chunk_bytes is None else chunk_bytes) // head_bytes)
     heads = min(H, max(heads_per_chunk, room))
     elements = min(E, max(1, room // H)) if heads == H else 1
     return heads, elements, max(1, room // 2)
 
 
-def plan_chunks(E: int, H: int, heads_per_chunk: int) -> list[tuple[int, int, int]]:
-    """(batch index, first head, number of heads) of every chunk, in the order the library runs them."""
+def plan_chunks(E: int, H: int, heads_per_chunk: int, elements_per_chunk: int = 1, least_heads: int = 1) -> list[tuple[int, int, int]]:
+    """(batch index, first head, number of heads, over whole elements where there are more than that element has left) of every
+    chunk, in the order the library runs them; the arguments are what ``group_chunks`` returns."""
     if E < 0 or H < 0:
         raise ValueError("E and H must be non-negative")
-    if heads_per_chunk < 1:
-        raise ValueError("heads_per_chunk must be at least 1")
-    out = []
-    for e in range(E):
-        h0 = 0
-        while h0 < H:
-            left = H - h0
-            nh = min(heads_per_chunk, left)
-            if e == E - 1 and nh > 1 and nh > left // 2:   # the last batch element tapers off
-                nh = max(1, left // 2)
-            out.append((e, h0, nh))
-            h0 += nh
-    return out
+    if min(heads_per_chunk, elements_per_chunk, least_heads) < 1:
+        raise ValueError("heads_per_chunk, elements_per_chunk and least_heads must be at least 1")
+    plan = _cabi.load().ma_b200_host_chunk_plan
+    n = plan(E, H, heads_per_chunk, elements_per_chunk, least_heads, None, 0)
+    flat = (C.c_int32 * (3 * n))()
+    plan(E, H, heads_per_chunk, elements_per_chunk, least_heads, flat, n)
+    return [tuple(flat[3 * i:3 * i + 3]) for i in range(n)]
 
 
 def monarch_attention_b200_host(q: Tensor, k: Tensor, v: Tensor, attn_mask: Tensor | None, T: int, B: int,
