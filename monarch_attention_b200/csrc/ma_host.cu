@@ -34,7 +34,7 @@ struct Pipes {
   // what the previous call on this device laid out in the scratch (a streamed call may only overlap a
   // previous call that used the same slots)
   const void* last_scratch = nullptr;
-  size_t last_slot_bytes = 0, last_total = 0;
+  size_t last_qk_bytes = 0, last_slot_bytes = 0, last_total = 0;
 };
 Pipes g_pipes[kMaxDevices];
 std::mutex g_pipes_mutex;
@@ -251,9 +251,10 @@ MA_B200_API int ma_b200_forward_host_grouped(const ma_b200_problem* p, int heads
   // copying out, provided that call used the scratch in the same way (same slots: the per-slot events then
   // order every reuse); anything else is ordered after what the caller has already queued on its stream,
   // which includes the end of the previous call.
-  const bool overlap = streamed != 0 && P->last_scratch == device_scratch && P->last_slot_bytes == L.slot_bytes &&
+  const bool overlap = streamed != 0 && P->last_scratch == device_scratch && P->last_qk_bytes == L.qk_bytes && P->last_slot_bytes == L.slot_bytes &&
                        P->last_total == L.total;
   P->last_scratch = device_scratch;
+  P->last_qk_bytes = L.qk_bytes;  // (a slot of the same size with its tensors elsewhere: copying in would run over a result on its way out)
   P->last_slot_bytes = L.slot_bytes;
   P->last_total = L.total;
   if (!overlap) {

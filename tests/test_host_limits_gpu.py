@@ -66,3 +66,21 @@ def test_chunks_over_elements_return_the_bits_of_one_device_call(chunk, layout, 
         out.zero_()
         ma.monarch_attention_b200_host(q, k, v, m, T, B, True, out=out, heads_per_chunk=1, chunk_bytes=chunk, streamed=streamed)
         assert torch.equal(out.contiguous().view(torch.int16), want.contiguous().view(torch.int16))
+
+
+@pytest.mark.gpu
+def test_streamed_calls_with_slots_of_one_size_and_other_tensors_in_them():
+    """Widths of 32 and 96 exchanged between q, k and v: the slots have one size, the results lie elsewhere in them."""
+    import monarch_attention_b200 as ma
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(11)
+    calls = []
+    for i in range(10):
+        D, Dv = (32, 96) if i % 2 else (96, 32)
+        q, k, v = (torch.randn(1, 8, 600, w, generator=g).to(torch.bfloat16).pin_memory() for w in (D, D, Dv))
+        calls.append((q, k, v, torch.empty_like(v).pin_memory()))
+    for q, k, v, out in calls:
+        ma.monarch_attention_b200_host(q, k, v, None, 1, 25, False, out=out, wait=False, streamed=True, heads_per_chunk=2)
+    torch.cuda.synchronize()
+    for q, k, v, out in calls:
+        assert torch.equal(out, ma.monarch_attention_b200(q.to(dev), k.to(dev), v.to(dev), None, 1, 25, False).cpu())
