@@ -26,6 +26,8 @@ _scratch: dict[int, Tensor] = {}
 # 1426, 1274, 1176, 1170; 8 of 8192 x 64, whose chunks are larger anyway, 699 / 679, 684, 667, 684.
 CHUNK_BYTES = 4 << 20
 HEADS_PER_CHUNK = 8
+# Most heads that the tensor-core kernels take in a launch (their grids' second dimension).
+GRID_HEADS = 65535
 
 
 def group_chunks(E: int, H: int, head_bytes: int, heads_per_chunk: int, chunk_bytes: int | None = None) -> tuple[int, int, int]:
@@ -33,8 +35,8 @@ def group_chunks(E: int, H: int, head_bytes: int, heads_per_chunk: int, chunk_by
     (default CHUNK_BYTES) of one tensor grows to that, over whole batch elements where it has all their heads, and is not cut to
     fewer than half of it at the end.  With 0 it is ``heads_per_chunk`` heads of one batch element."""
     room = -(-(CHUNK_BYTES if chunk_bytes is None else chunk_bytes) // head_bytes)
-    heads = min(H, max(heads_per_chunk, room))
-    elements = min(E, max(1, room // H)) if heads == H else 1
+    heads = min(H, max(heads_per_chunk, min(room, GRID_HEADS)))
+    elements = min(E, max(1, min(room, GRID_HEADS) // H)) if heads == H else 1
     return heads, elements, max(1, room // 2)
 
 

@@ -40,3 +40,9 @@ def test_every_head_is_in_one_chunk():
         per_element = -(-H // heads)
         full = -(-E // elements) if elements > 1 else E * per_element
         assert len(plan) <= full + H.bit_length()
+
+
+def test_a_chunk_is_no_larger_than_a_grid():
+    for E, H in ((200000, 1), (3, 70000), (9000, 30)):
+        heads, elements, _ = group_chunks(E, H, 16, 8)
+        assert heads * elements <= 65535

@@ -84,3 +84,15 @@ def test_streamed_calls_with_slots_of_one_size_and_other_tensors_in_them():
     torch.cuda.synchronize()
     for q, k, v, out in calls:
         assert torch.equal(out, ma.monarch_attention_b200(q.to(dev), k.to(dev), v.to(dev), None, 1, 25, False).cpu())
+
+
+@pytest.mark.gpu
+def test_more_heads_than_a_grid_takes():
+    """In chunks each family runs any number of heads: here one that is asked for by name, of one token each."""
+    import monarch_attention_b200 as ma
+    from monarch_attention_b200 import _cabi
+    E, H = 9000, 8
+    g = torch.Generator().manual_seed(1)
+    q, k, v = (torch.randn(E, H, 1, 8, generator=g).to(torch.bfloat16).pin_memory() for _ in range(3))
+    out = ma.monarch_attention_b200_host(q, k, v, None, 1, 1, False, kernel=_cabi.KERNEL_WARP_MMA)
+    assert torch.equal(out, v)  # (one token attends to itself)
