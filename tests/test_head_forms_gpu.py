@@ -25,3 +25,20 @@ def test_forms_give_the_same_bits(H, B, M, D, T, masked, dtype):
     some = [t[:, 50:50 + H] for t in (q, k, v)]
     for _ in range(2):
         assert torch.equal(mod(*some, m), want[:, 50:50 + H])
+
+
+@pytest.mark.parametrize("D", range(8, 81, 8))
+def test_every_shape_has_a_kernel(D):
+    """Sides and numbers of heads around all lines of the choice; with every row of v equal to c, every row of the result is c."""
+    import monarch_attention_b200 as ma
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k = (torch.randn(1, 160, 32 * 32, D, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    c = torch.linspace(-2, 2, D, device="cuda").to(torch.bfloat16)
+    v = c.expand(1, 160, 32 * 32, D).contiguous()
+    for B in (1, 16, 17, 24, 25, 32):
+        for M in (1, 16, 17, 24, 25, 32):
+            for H in (1, 33, 40, 75, 91, 148, 160):
+                for T in (1, 2):
+                    out = ma.MonarchAttention(B, T, "post", impl="b200-head-resident")(*(t[:, :H, :B * M] for t in (q, k, v)))
+                    # (factors and y are rounded to 8 bits of mantissa: up to 2 ulp of 2 in the sum)
+                    assert (out.float() - c.float()).abs().max().item() < 3e-2, (B, M, H, T)
