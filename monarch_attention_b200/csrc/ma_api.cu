@@ -87,22 +87,21 @@ ma::Geometry make_geometry(const ma_b200_problem* p, int mask_type = MA_B200_MAS
 
 // Whether the warp-level kernels are expected to take a problem faster than the tcgen05 tile kernels: those work on tiles of
 // 128 x 64 or 128 x 128 whatever the blocks fill of them, so that blocks just above 32, a long side beside a short one,
-// narrow heads and few heads are better off with 16-row warps and two launches.  Microseconds of one iteration, from a
-// sweep of blocks and counts of 16 to 200, 4 to 256 heads and widths 32 and 64: a tile takes 12.5 ns of the GPU's time and an
-// iteration 18.6 us at the least (8 beside the tiles' own time); a padded element of a warp-level tile takes 2.4 ps (1.7 in
-// heads of up to 32), two launches 6 us.  Measured again with the single-launch tile kernels' split roles, both families on blocks and
-// counts of 8 to 128, 4 to 256 heads, one and two iterations (675 calls): what the rule takes sums up to 0.5 % more than the
-// faster one of each call, and 23 calls lose more than 5 %: 128 x 16 x 64 the most, us, warp-level / tile with one iteration 52 / 43 at
-// 48 heads, 125 / 93 at 128, 239 / 173 at 256; 96 x 33 x 32 the other way, 22.8 / 26.9 at 16.
+// narrow heads and few heads are better off with 16-row warps and two launches.  Microseconds of one iteration, fitted to 1008 pairs
+// of calls (36 shapes of 8 to 128, widths 32 and 64, 4 to 256 heads, one and two iterations, replayed from a graph): a tile takes 8.2 ns of
+// the GPU's time beside 10.9 us; a padded element of a warp-level tile, keys and rows to the next multiple of 16, takes 3.13 ps in the
+// right-factor stage and 1.62 in the left-factor or output stage, 0.55 of that in heads of up to 32, beside 3.8 us.  What the rule takes
+// is 0.1 % more than the faster one of each pair as a geometric mean, and 11 pairs lose more than 5 %: us, warp-level / tile, 96 heads of
+// 96 x 33 x 32, two iterations, 171 / 150 the most that is lost by the warp-level kernels, 16 of 49 x 49 x 64 34.9 / 39.9 by the tiles.
+// (Before, keys counted as 16, 32, 64 or 128, as the kernels once padded them, and one cost for both stages: 1.9 % and 123 pairs; 4 heads
+// of 72 x 72 x 64, one iteration, 12.4 / 18.5 and 128 of 128 x 16 x 64 122 / 89 were on the wrong side.)
 bool warp_beats_tiles(const ma::Geometry& g, double heads) {
   if (g.B > 128 || g.M > 128) return false;  // (the warp-level kernels then walk a row twice: never the faster ones)
-  auto up16 = [](int x) { return (x + 15) & ~15; };
-  auto keys = [](int x) { return x <= 16 ? 16 : x <= 32 ? 32 : x <= 64 ? 64 : 128; };
-  const double elements = heads * ((double)g.M * up16(g.B) * keys(g.B) + (double)g.B * up16(g.M) * keys(g.M));
+  auto padded = [](int x) { return (double)((x + 15) & ~15); };
+  const double right = heads * g.M * padded(g.B) * padded(g.B), left = heads * g.B * padded(g.M) * padded(g.M);
   const double tiles = heads * ((g.B <= 64 ? (g.M + 1) / 2 : g.M) + (g.M <= 64 ? (g.B + 1) / 2 : g.B));
-  const double warp_us = 6.0 + elements * (g.D <= 32 ? 1.7e-6 : 2.4e-6);
-  const double tile_us = tiles * 12.5e-3 + 8.0;
-  return warp_us < (tile_us > 18.6 ? tile_us : 18.6);
+  const double warp_us = 3.8 + (3.13e-6 * right + 1.62e-6 * left) * (g.D <= 32 ? 0.55 : 1.0);
+  return warp_us < tiles * 8.2e-3 + 10.9;
 }
 
 // AUTO goes by the shape of a head and by how many heads there are.  `heads`: the (batch, head) pairs of the whole call, of
@@ -138,20 +137,19 @@ int resolve_kernel(const ma_b200_problem* p, const ma::Geometry& g, long long he
   const bool tf32_pays = tf32_ok && g.D >= 24;
   // The fused kernel takes one tile at a time through an SM, quickly; the tile kernels take four, each more slowly, and do
   // 1.2 to 1.4 times as many in a time.  So the fused kernel is the faster one while a stage is few rounds of one tile per
-  // SM.  Measured (us, fused / tile kernels, calls back to back on three sets of inputs) over 128 to 1536 tiles per stage, blocks
-  // of 64 and 128: with two iterations 42.0 / 44.0 and 47.1 / 51.6 at 3.5 tiles per SM, 49.7 / 50.6 and 59.2 / 62.3 at 5.2, 53.4 /
-  // 51.8 (blocks of 64) at 5.6, 57.3 / 52.9 and 68.2 / 65.0 at 6.1, 77 / 55 and 76 / 69 at 6.9; with three 69.8 / 69.6 and 82 / 90 at
-  // 5.2, 73.9 / 70.1 (64) at 5.6, 79 / 72 and 95 / 94 at 6.1: the line is at 5.5.  With one, whose two stages leave the tile kernels'
-  // list fewer waits, 16.5 / 18.5 and 18.5 / 18.7 at 0.9, 20.4 / 19.3 and 21.3 / 20.8 at 1.7, 22.7 / 21.8 and 24.9 / 24.7 at 2.6: the
-  // line at 2 was drawn before the roles of the tile kernels were split, and takes up to 5 % too long between 1 and 2.
+  // SM.  Measured (us, fused / tile kernels, replayed from a graph, both with their programmatic launches) over 0.4 to 8.7 tiles per SM
+  // and stage, blocks of 64 and 128: with two iterations 38.9 / 41.6 and 43.4 / 48.1 at 3.5, 47.3 / 48.8 and 55.5 / 57.0 at 5.2, 48.5 / 49.6
+  // (blocks of 64) at 5.4, 50.4 / 49.8 at 5.6, 54.1 / 50.8 and 65.2 / 61.6 at 6.1, 74 / 52 and 72 / 65 at 6.9; with three 66.5 / 67.3 and 79 / 87 at
+  // 5.2, 68.5 / 67.7 at 5.4, 75.8 / 69.0 and 91.7 / 91.2 at 6.1: the line is at 5.5.  With one, whose two stages leave the tile kernels' list
+  // fewer waits, 14.1 / 15.9 and 15.5 / 17.6 at 0.9, 17.2 / 17.7 and 18.8 / 19.9 at 1.7, 19.6 / 18.9 at 2.2, 21.0 / 20.0 and 23.2 / 22.4 at 2.6: the
+  // line is at 2.
   const bool few_tiles = tc_ok && heads * p->N / 64 <= (long long)ma::sm_count() * (p->num_steps == 1 ? 4 : 11);
   // Head widths other than 32, 64, 72 and 80 have one tile size for both kinds of stage in the head-resident kernel: with one side of
   // up to 16 beside a longer one the warp-level kernels pad less, and win once the heads no longer fit the SMs in one round.
-  // Measured before 32 and 80 had tiles of their own (us, head-resident / warp-level; blocks of 8 x 20 to 16 x 24, one and two
-  // iterations), 10 x 30 x 80 with two: 33 / 37 at 148 heads, 60 / 39 at 160, 88 / 62 at 300, 124 / 115 at 592; 10 x 30 x 32 with one:
-  // 13 / 16, 21 / 17, 32 / 23, 39 / 37.  With tiles of their own, head-resident / warp-level: 10 x 30 x 32 with one 10.7 / 14.6 at 160, 17.5 /
-  // 19.7 at 300, 25.2 / 34.2 at 592, 16 x 24 x 32 with two 18.1 / 27.9, 28.6 / 42.1, 38.7 / 74.8; 10 x 30 x 80 with two 34.0 / 37.4, 54.6 /
-  // 58.8, 77.0 / 112.  Width 80 is still on the other side of this line, since parts of calls are held to the family it gives.
+  // Head-resident over warp-level, 112 calls each (8 x 20 to 32 x 5, 149 to 1000 heads, one and two iterations, replayed from a graph): width
+  // 40 1.24 as a geometric mean (10 x 30, one iteration, 149 heads 1.64; 16 x 17, two, 592 heads 0.88), 48 1.25, 56 1.26, 24 1.12.  Width 80, with
+  // tiles of its own, 0.81 (1.05 the most, 300 heads of 16 x 17 with one) would be faster on the other side of this line; it stays because
+  // test_parts_gpu.py needs a part of 200 heads of 10 x 30 x 80 to be of another family than the whole.
   const bool lopsided = (g.B <= 16) != (g.M <= 16) && g.D != 32 && g.D != 64 && g.D != 72 && heads > ma::sm_count();
   if (p->kernel == MA_B200_KERNEL_AUTO)
     *kernel = few_tiles ? MA_B200_KERNEL_TCGEN05
