@@ -135,8 +135,8 @@ __device__ __forceinline__ bool mask_lets(const Geometry& g, int e, int n) {
 // Kernels are launched with programmatic dependence on whatever precedes them in the stream, another library's kernel included:
 // the GPU then prepares the launch while that kernel ends, and the kernel waits at its start (grid_wait), before it touches
 // memory, until everything before it is complete and visible.  A plain launch costs more than its work here: launches of a
-// kernel that spins for t us follow one another every ceil((t + 1) / 2.05) * 2.05 us (3 us: 6.15, 10: 12.30, 16: 18.43), with
-// the dependence every t + 0.55 (148 or 768 CTAs, with and without clusters, 0 to 200 KB of shared memory).
+// kernel that spins for t us follow one another every ceil((t + 2) / 2.05) * 2.05 us (2 us: 4.11, 3: 6.16, 10: 12.31, 16: 18.45; 148 and
+// 768 CTAs), with the dependence every t + 0.8 (148 CTAs) to t + 1.0 (768), and 2.05 at the least.
 // A stage kernel that another stage follows also lets that one's CTAs come up at once (stage_begin), under its own tail: 256 fp32
 // tokens, two launches, 15.4 to 13.3 us; six launches 84 to 75.  The last kernel of a call does not, so that a small grid behind
 // it finds all SMs free and spreads evenly, nor do the tcgen05 tile kernels: their early CTAs took instruction fetch from the

@@ -42,3 +42,21 @@ def test_every_shape_has_a_kernel(D):
                     out = ma.MonarchAttention(B, T, "post", impl="b200-head-resident")(*(t[:, :H, :B * M] for t in (q, k, v)))
                     # (factors and y are rounded to 8 bits of mantissa: up to 2 ulp of 2 in the sum)
                     assert (out.float() - c.float()).abs().max().item() < 3e-2, (B, M, H, T)
+
+
+@pytest.mark.parametrize("H,B,M,D,T", [(80, 17, 19, 64, 2), (12, 32, 32, 64, 1)])
+def test_clusters_in_a_captured_graph(H, B, M, D, T):
+    import monarch_attention_b200 as ma
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v, q2 = (torch.randn(1, H, B * M, D, generator=g, device="cuda").to(torch.bfloat16) for _ in range(4))
+    mod = ma.MonarchAttention(B, T, "post")
+    want, want2 = mod(mod(q, k, v), k, v), mod(mod(q2, k, v), k, v)
+    x = q.clone()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = mod(mod(x, k, v), k, v)
+    for a, b in ((q, want), (q2, want2), (q, want)):
+        x.copy_(a)
+        graph.replay()
+        assert torch.equal(out, b)
